@@ -540,8 +540,10 @@ def main():
     it_fp64 = paths["fp64"]["iterations"]
 
     # roofline of the T2 update kernel (mixed, FP32 storage, DIIS ring write)
+    # of the problem that runs: one channel when the labels are alike
     n_t2 = plan.n_t2
-    alg_bytes = (3 * n_t2 + eng.n_g) * 4
+    work = eng.reduced() or eng
+    alg_bytes = (3 * work.plan.n_t2 + work.n_g) * 4
     k_ms = statistics.mean(m_k)
     achieved = alg_bytes / (k_ms * 1e-3) / 1e9
     peaks = {}
@@ -563,7 +565,7 @@ def main():
            "scaling": "weak", "vs_baseline": None, "dtype": "f32+f64",
            "data": "synthetic: lattice Hamiltonian built in-process (no dataset)",
            "config": {"workload": "ccsd_L6_A28_mixed", "L": L_BENCH, "A": A_BENCH, "p": plan.p, "h": plan.h,
-                      "C2": C2, "C3": C3, "units": "hbar^2/(M a^2)", "n_t2_compact": n_t2,
+                      "C2": C2, "C3": C3, "units": "hbar^2/(M a^2)", "n_t2_compact": n_t2, "n_t2_stored": work.plan.n_t2,
                       "tune": {"word": int(eng.prob.tune), "choice": T.describe(int(eng.prob.tune)),
                                "cached": tune_info.get("cached")},
                       "max_diis": 8, "mixed_eps": 1e-8, "refine": refine,

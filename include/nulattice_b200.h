@@ -71,7 +71,12 @@ typedef struct {
                                        pass: 5 256x1, 6 384x1, 7 448x1, 8 512x1);
                                      bits 4-7 lattice Lambda row pass, FP32 (0 256x2, 1 512x1);
                                      bits 8-15 Lambda column-pass row chunks (0: automatic);
-                                     bits 16-19 lattice T2 kernel, FP64 (0 512x1, 1 256x1) */
+                                     bits 16-19 lattice T2 kernel, FP64 (0 512x1, 1 256x1);
+                                     bits 24-31 alike labels m (0 or 1: every label is stored).  m > 1:
+                                       the m labels have the same tables, ladders and amplitudes, and
+                                       every pair of labels the same exchange-symmetric t2; the problem
+                                       stores one label and its one channel (g1 = g2 = 0), t1 [p*h] of
+                                       that label, and energies, norms and DIIS weights count all m */
     const nlb_channel *chan;      /* [n_channels] */
     const int64_t *t2_end;        /* [n_channels] cumulative end of each block */
     const int64_t *g_end;         /* [n_channels] cumulative end of Ga blocks */
@@ -220,6 +225,24 @@ int nlb_struct_unpack_t2(const nlb_struct_problem *prob, const void *t2c, int32_
                          double *t2_dense, nlb_stream_t stream);
 int nlb_struct_pack_t2(const nlb_struct_problem *prob, const double *t2_dense, void *t2c,
                        int32_t dtype, nlb_stream_t stream);
+
+/* Label-symmetric problems (tune bits 24-31; prob is the stored label's).
+ * p_ord / h_ord list the particles / holes of all m labels, label by label,
+ * each label in the stored label's order.
+ *
+ * nlb_sym_check: do amplitudes of the full layout (t1 [mp * mh], compact t2 of
+ * all pairs of labels) have the symmetric form?  out (device, 3 words):
+ * [0] != 0 when labels differ; [1], [2] the bits of the largest
+ * |B[a,b,i,j] - B[b,a,j,i]| and |B[a,b,i,j]| of the first block.  t1_out
+ * (optional, [p*h]) receives t1 of the first label.
+ * nlb_sym_expand: the full layout from the stored parts: t1 (or NULL), and t2
+ * (or NULL) as copies of the block for every pair (compact, same dtype) or,
+ * dense != 0, as the FP64 tensor t2[a,b,i,j] (zero-filled by the caller). */
+int nlb_sym_check(const nlb_struct_problem *prob, const int32_t *p_ord, const int32_t *h_ord, const double *t1,
+                  const void *t2, int32_t dtype, double *t1_out, uint64_t *out, nlb_stream_t stream);
+int nlb_sym_expand(const nlb_struct_problem *prob, const int32_t *p_ord, const int32_t *h_ord, const double *t1,
+                   double *t1_full, const void *t2, int32_t dtype, void *t2_full, int32_t dense,
+                   nlb_stream_t stream);
 
 /* ---------------------------------------------------------------------
  * Adjoint of the structured engine (no counterpart in the reference, which

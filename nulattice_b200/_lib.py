@@ -155,6 +155,11 @@ def lib():
     L.nlb_struct_step_noalloc.restype = c_int32
     L.nlb_struct_noalloc_scratch_bytes.argtypes = [ctypes.POINTER(StructProblem), c_int32]
     L.nlb_struct_noalloc_scratch_bytes.restype = c_int64
+    L.nlb_sym_check.argtypes = [ctypes.POINTER(StructProblem), c_void_p, c_void_p, c_void_p, c_void_p, c_int32,
+                                c_void_p, c_void_p, c_void_p]
+    L.nlb_sym_expand.argtypes = [ctypes.POINTER(StructProblem), c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                 c_int32, c_void_p, c_int32, c_void_p]
+    L.nlb_sym_check.restype = L.nlb_sym_expand.restype = c_int32
     for name in ("nlb_struct_ctrl_init", "nlb_struct_step", "nlb_struct_diis", "nlb_struct_energy",
                  "nlb_convert", "nlb_struct_unpack_t2", "nlb_struct_pack_t2"):
         getattr(L, name).restype = c_int32

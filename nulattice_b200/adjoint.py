@@ -34,7 +34,10 @@ def diag_coefficients(eng, dtwo):
     """Map a derivative Hamiltonian's v_hhhh / v_pppp onto the engine's
     channels as diagonal ladder coefficients (dw, dv), laid out like the
     hole-hole / particle-particle CSR pointer arrays."""
-    pl = eng.plan
+    return _diag_coefficients(eng.plan, dtwo)
+
+
+def _diag_coefficients(pl, dtwo):
     hh_idx, hh_val = _structure._coo(dtwo[5])
     pp_idx, pp_val = _structure._coo(dtwo[0])
     dw = np.zeros(max(sum(len(x) for x in pl.hh_ptr), 1))
@@ -60,31 +63,63 @@ def diag_coefficients(eng, dtwo):
     return dw, dv
 
 
+def _label_coefficients(eng, dfock, dtwo):
+    """(dw, dv, df_hh) of one label of a reduced engine, None when the
+    derivative Hamiltonian treats the labels differently."""
+    pl = eng.full_plan
+    dw, dv = _diag_coefficients(pl, dtwo)
+    n = len(pl.channels)
+    nw, nv = len(pl.hh_ptr[0]), len(pl.pp_ptr[0])
+    dw, dv = dw.reshape(n, nw), dv.reshape(n, nv)
+    df = np.asarray(dfock[2], dtype=np.float64)
+    blocks = [df[np.ix_(H, H)] for H in pl.h_of]
+    if any(not np.array_equal(x, dw[0]) for x in dw) or any(not np.array_equal(x, dv[0]) for x in dv) or \
+            any(not np.array_equal(x, blocks[0]) for x in blocks) or \
+            np.count_nonzero(df) != len(blocks) * np.count_nonzero(blocks[0]):
+        return None
+    return dw[0], dv[0], blocks[0]
+
+
 class LambdaSolver:
     """Buffers and captured step graphs of the Lambda iteration for one
-    engine (kept on the engine, so repeated gradients reuse them)."""
+    engine (kept on the engine, so repeated gradients reuse them).
+
+    When the engine's labels are alike and the amplitudes handed to
+    :meth:`run` have that form, the iteration runs on one label and its
+    multipliers, U, T and control block are written out in the layout of the
+    full buffers."""
 
     def __init__(self, eng):
         L = _lib.lib()
         self.eng = eng
         self.lattice = bool(L.nlb_lambda_lattice(eng.prob))
         self.n_gb = int(L.nlb_lambda_gb_len(eng.prob))
+        self._label = None
         self._bufs = {}
         self._coef = {}
 
     def coefficients(self, dfock, dtwo):
         """Device (dw, dv) and the host f_hh block of a derivative
-        Hamiltonian, mapped and checked once (its f_pp and f_ph must vanish)."""
+        Hamiltonian, mapped and checked once (its f_pp and f_ph must vanish).
+        On a one-label engine: those of one label, None when they differ."""
         key = (id(dfock), id(dtwo))
         if key not in self._coef:
             df_pp, df_ph, df_hh = [np.asarray(f) for f in dfock]
             if np.any(df_pp) or np.any(df_ph):
                 raise ValueError("derivative Fock blocks f_pp/f_ph must vanish (closed-site inputs)")
-            dw, dv = diag_coefficients(self.eng, dtwo)
+            if self.eng.labels > 1:
+                got = _label_coefficients(self.eng, dfock, dtwo)
+                if got is None:
+                    self._coef[key] = (dfock, dtwo, None)
+                    return None
+                dw, dv, df_hh = got
+            else:
+                dw, dv = diag_coefficients(self.eng, dtwo)
             dev = self.eng.dev
             self._coef[key] = (dfock, dtwo, torch.as_tensor(dw, dtype=torch.float64, device=dev),
                                torch.as_tensor(dv, dtype=torch.float64, device=dev), np.array(df_hh, dtype=np.float64))
-        return self._coef[key][2:]
+        got = self._coef[key]
+        return None if got[2] is None else got[2:]
 
     def buffers(self, dtype_code, max_diis):
         key = (dtype_code, max_diis)
@@ -146,6 +181,9 @@ class LambdaSolver:
 
     def run(self, b, tol, mixing, max_steps, max_diis, keep):
         """Iterate to the relative step tol; returns the final ctrl block."""
+        label = self._alike(b, keep)
+        if label is not None:
+            return self._run_label(label, b, tol, mixing, max_steps, max_diis, keep)
         L = _lib.lib()
         dev = self.eng.dev
         stream = torch.cuda.current_stream(dev)
@@ -172,6 +210,44 @@ class LambdaSolver:
         return c
 
 
+    def _alike(self, b, keep):
+        """(one-label solver, its start) when the amplitudes of ``b`` (and the
+        multipliers, if kept) have the alike-label form, else None."""
+        red = self.eng.reduced()
+        if red is None:
+            return None
+        t1 = red.compress(b["t1"], b["t2"])
+        lam1 = red.compress(b["lam1"][0], b["lam2"][0]) if keep and t1 is not None else None
+        if t1 is None or (keep and lam1 is None):
+            return None
+        if self._label is None:
+            self._label = LambdaSolver(red)
+        return self._label, t1, lam1
+
+    def _run_label(self, label, b, tol, mixing, max_steps, max_diis, keep):
+        solver, t1, lam1 = label
+        red = solver.eng
+        n, p, h = red.plan.n_t2, red.plan.p, red.plan.h
+        r = solver.buffers(b["state"].dtype, max_diis)
+        r["t1"].copy_(t1)
+        r["t2"].copy_(b["t2"][:n])
+        if keep:
+            r["lam1"][0].copy_(lam1)
+            r["lam2"][0].copy_(b["lam2"][0][:n])
+        c = solver.run(r, tol, mixing, max_steps, max_diis, keep)
+        cur = c.parity
+        red._expand(r["lam1"][cur], b["lam1"][cur], r["lam2"][cur], b["lam2"][cur], False)
+        # U and T of every label behind the Z1 accumulator, as in the full layout
+        P, H = red.sizes
+        ut = torch.zeros((2, H, H), dtype=torch.float64, device=red.dev)
+        idx = red.orders[1].long().reshape(red.labels, h)
+        ut[:, idx[:, :, None], idx[:, None, :]] = r["acc"][p * h:p * h + 2 * h * h].reshape(2, 1, h, h)
+        b["acc"][P * H:P * H + 2 * H * H].copy_(ut.reshape(-1))
+        b["ctrl"].copy_(r["ctrl"])
+        self.launches = solver.launches + 2
+        return c
+
+
 def lambda_gradient(eng, t1_dev, t2c_dev, derivs, tol=1e-9, mixing=0.5, max_steps=5000, max_diis=8,
                     precision="mixed", tol_fp32=1e-6, info=None):
     """Solve the Lambda equations at (t1, compact t2) and return dE/dc for each
@@ -183,13 +259,22 @@ def lambda_gradient(eng, t1_dev, t2c_dev, derivs, tol=1e-9, mixing=0.5, max_step
     subspace (0: plain Jacobi with mixing)."""
     info = {} if info is None else info
     L = _lib.lib()
+    red = eng.reduced()
+    if not (red or eng).prob.diag_ladders:
+        raise ValueError("the adjoint needs diagonal ladders (SU(4) closed-site inputs)")
+    if red is not None:
+        # alike labels: everything on one of them, when the amplitudes and the
+        # derivative Hamiltonians treat the labels alike, too
+        solver = _kept_solver(red)
+        t2c_dev = t2c_dev.reshape(-1).contiguous()
+        t1 = None
+        if all(solver.coefficients(dfock, dtwo) is not None for _, dfock, dtwo in derivs):
+            t1 = red.compress(t1_dev.to(torch.float64).contiguous(), t2c_dev)
+        if t1 is not None:
+            eng, t1_dev, t2c_dev = red, t1, t2c_dev[:red.plan.n_t2]
     pl, dev = eng.plan, eng.dev
     sp = ctypes_void(torch.cuda.current_stream(dev).cuda_stream)
-    if not eng.prob.diag_ladders:
-        raise ValueError("the adjoint needs diagonal ladders (SU(4) closed-site inputs)")
-    solver = getattr(eng, "_lambda_solver", None)
-    if solver is None:
-        solver = eng._lambda_solver = LambdaSolver(eng)
+    solver = _kept_solver(eng)
     if not solver.lattice:
         precision, max_diis = "fp64", max_diis   # the general path iterates in FP64
     torch.cuda.synchronize(dev)
@@ -238,7 +323,7 @@ def lambda_gradient(eng, t1_dev, t2c_dev, derivs, tol=1e-9, mixing=0.5, max_step
                                          out[n:].data_ptr(), sp), "lambda_coupling")
         launches += 1
     outn = out.cpu().numpy()
-    grads = [float(de_ref) - float(np.sum((U + T) * df_hh)) + float(outn[n])
+    grads = [float(de_ref) - eng.labels * float(np.sum((U + T) * df_hh)) + float(outn[n])
              for n, ((de_ref, _, _), (_, _, df_hh)) in enumerate(zip(derivs, coefs))]
     torch.cuda.current_stream(dev).synchronize()
     info.update(lambda_status=status, lambda_iters=iters, t_lambda=time.perf_counter() - t0,
@@ -247,6 +332,13 @@ def lambda_gradient(eng, t1_dev, t2c_dev, derivs, tol=1e-9, mixing=0.5, max_step
     if status != "converged":
         raise RuntimeError(f"Lambda equations did not converge: {status}")
     return grads
+
+
+def _kept_solver(eng):
+    solver = getattr(eng, "_lambda_solver", None)
+    if solver is None:
+        solver = eng._lambda_solver = LambdaSolver(eng)
+    return solver
 
 
 _PROBLEMS = {}
@@ -291,7 +383,7 @@ def ccsd_energy_and_gradient(L, holes, C2, C3, device="cuda:0", precision="fp64"
             raise ValueError(f"the adjoint needs the structured engine: {why}")
         engine = StructuredEngine(plan, fock, dev)
         from . import tune as _tune
-        engine.prob.tune = _tune.known_word(engine)
+        engine.tune = _tune.known_word(engine)
     eng = info["engine"] = engine
     torch.cuda.synchronize(dev)
     t0 = time.perf_counter()

@@ -143,13 +143,22 @@ class _Instance:
         plan, why = _structure.detect(fock, two)
         if plan is None:
             raise ValueError(f"instance (A={A}, L={L}) needs the structured engine: {why}")
-        self.eng = eng = StructuredEngine(plan, fock, dev)
+        self.eng = StructuredEngine(plan, fock, dev)
+        # alike labels: the instance runs on one of them
+        solver = None
+        eng = self.eng.reduced()
+        if eng is not None:
+            solver = _adj.LambdaSolver(eng)
+            if any(solver.coefficients(x[1], x[2]) is None for x in (prob.dv, prob.dw)):
+                eng = None
+        if eng is None:
+            eng, solver = self.eng, _adj.LambdaSolver(self.eng)
+        self.work = eng
         self.lattice = bool(L_.nlb_lambda_lattice(eng.prob))
-        f_pp, f_ph, f_hh = [np.asarray(f) for f in fock]
-        t1 = _mp2_t1(f_pp, f_ph, f_hh, 0.0)
-        self.e0 = float(np.sum(f_ph * t1))
-        self.t1_init = torch.as_tensor(t1.reshape(-1), device=dev)
-        pl = plan
+        t1 = _mp2_t1(eng.f_pp_np, eng.f_ph_np, eng.f_hh_np, 0.0)
+        self.e0 = eng.labels * float(np.sum(eng.f_ph_np * t1))
+        self.t1_init = torch.as_tensor(np.ascontiguousarray(t1).reshape(-1), device=dev)
+        pl = eng.plan
         n1, n2 = pl.p * pl.h, max(pl.n_t2, 1)
         self.f32 = eng.buffers(_lib.NLB_F32, max_diis)
         self.f64 = eng.buffers(_lib.NLB_F64, max_diis)
@@ -173,8 +182,8 @@ class _Instance:
         self.l64 = lam_buffers(torch.float64, own_t2=False)
         self.l32 = lam_buffers(torch.float32, own_t2=True) if self.lattice else None
         self.out = torch.zeros(8, **f64)
-        solver = _adj.LambdaSolver(eng)
-        self.dw_dv = [solver.coefficients(prob.dv[1], prob.dv[2])[:2], solver.coefficients(prob.dw[1], prob.dw[2])[:2]]
+        coef = [solver.coefficients(x[1], x[2]) for x in (prob.dv, prob.dw)]
+        self.dw_dv, self.df_hh = [c[:2] for c in coef], [c[2] for c in coef]
 
     def lambda_state(self, b, dtype, fwd, ring):
         st = _lib.LambdaState()
@@ -191,7 +200,8 @@ class _Instance:
 
     def item(self):
         it = _lib.BatchItem()
-        it.prob = ctypes.pointer(self.eng.prob)
+        self.work.tune = self.eng.tune
+        it.prob = ctypes.pointer(self.work.prob)
         it.f32 = self.f32["state"]
         it.f64 = self.f64["state"]
         it.l64 = self.lambda_state(self.l64, _lib.NLB_F64, self.f64, self.f64)
@@ -226,8 +236,8 @@ class BatchScan:
                 if cls not in self.tuning:
                     info = {}
                     _tune.tune(x.eng, info=info)
-                    self.tuning[cls] = (int(x.eng.prob.tune), info)
-                x.eng.prob.tune = self.tuning[cls][0]
+                    self.tuning[cls] = (x.eng.tune, info)
+                x.eng.tune = self.tuning[cls][0]
         items = (_lib.BatchItem * len(self.instances))(*[x.item() for x in self.instances])
         self._items = items
         cfg = _lib.BatchConfig(mixing=mixing, mixed_eps=mixed_eps, eps=eps, lambda_tol_fp32=lambda_tol_fp32,
@@ -254,20 +264,18 @@ class BatchScan:
         status = {0: "running", 1: "converged", 2: "max_iter", 3: "diverged"}
         for x in self.instances:
             o = x.out.cpu().numpy()
-            pl = x.eng.plan
-            p, h = pl.p, pl.h
+            p, h = x.work.plan.p, x.work.plan.h
             ut = x.l64["acc"][p * h:p * h + 2 * h * h].cpu().numpy()   # U and T only
             UT = ut[:h * h].reshape(h, h) + ut[h * h:].reshape(h, h)
             grads = []
             ok = int(o[5]) == 1   # the Lambda equations converged (the forward solve did, too)
             for d, part in enumerate((x.prob.dv, x.prob.dw)):
-                de_ref, dfock = part[0], part[1]
-                g = 2.0 * (float(de_ref) - float(np.sum(UT * np.asarray(dfock[2]))) + float(o[1 + d]))
+                g = 2.0 * (float(part[0]) - x.work.labels * float(np.sum(UT * x.df_hh[d])) + float(o[1 + d]))
                 grads.append(g if ok else float("nan"))
             res.append(dict(A=x.A, L=x.L, C2=x.C2, C3=x.C3, E=float(o[0]) + x.e_ref, E_corr=float(o[0]),
                             dE_dC2=grads[0], dE_dC3=grads[1], status=status.get(int(o[3]), "?"),
                             lambda_status=status.get(int(o[5]), "?"), iterations=int(o[4]),
-                            mixed_iterations=int(o[7]), lambda_iterations=int(o[6]), n_t2=pl.n_t2))
+                            mixed_iterations=int(o[7]), lambda_iterations=int(o[6]), n_t2=x.eng.plan.n_t2))
         return res
 
     def close(self):

@@ -80,15 +80,131 @@ class StructuredEngine:
 
     Building it uploads the channel plan once; :meth:`solve` can then be
     called repeatedly (different initial amplitudes, precision, tolerances).
+
+    When the labels are alike (:func:`structure.alike_labels`), the work runs
+    on :meth:`reduced`, the engine of one label and one channel, and the
+    results are written out in the full layout; the tables of the full
+    problem are then built when something asks for them (``prob``).
+
+    ``labels``: how many alike labels a one-label plan stands for.
     """
 
-    def __init__(self, plan, fock_mats, device):
+    def __init__(self, plan, fock_mats, device, labels=1):
         self.plan = plan
         self.dev = device
+        self.labels = labels
         f_pp, f_ph, f_hh = [np.asarray(_np(f), dtype=np.float64) for f in fock_mats]
         self.f_ph_np = f_ph
         self.f_pp_np, self.f_hh_np = f_pp, f_hh
-        pl = plan
+        chs = plan.channels
+        self.n_g = sum(ch.nh1 * ch.np2 * ch.nh1 * ch.nh2 for ch in chs)
+        self.n_f2 = sum(ch.np1 * ch.nh1 for ch in chs)
+        self.n_rows = sum(ch.np1 for ch in chs)
+        self._prob = None
+        self._tune = 0
+        self._bufs = {}
+        self.cache = {}
+        self.launches = 0
+
+    @property
+    def prob(self):
+        """The device problem (:c:type:`nlb_struct_problem`), built on first use."""
+        if self._prob is None:
+            self._build()
+        return self._prob
+
+    @property
+    def tables(self):
+        self.prob
+        return self._tables
+
+    @property
+    def tune(self):
+        """The tuning word (launch shapes) of the problem."""
+        return self._tune if self._prob is None else int(self._prob.tune) & 0xffffff
+
+    @tune.setter
+    def tune(self, word):
+        self._tune = int(word) & 0xffffff
+        if self._prob is not None:
+            self._prob.tune = self._tune_word()
+
+    def _tune_word(self):
+        w = self._tune | ((self.labels << 24) if self.labels > 1 else 0)
+        return w - (1 << 32) if w >= 1 << 31 else w
+
+    def reduced(self):
+        """The engine of one label (None unless the labels are alike), with the
+        flags that were set on this engine's problem."""
+        if self.labels > 1:
+            return None
+        if "reduced" not in self.cache:
+            red = None
+            got = _structure.alike_labels(self.plan, self.f_hh_np)
+            if got is not None:
+                one, m = got
+                P0, H0 = self.plan.p_of[0], self.plan.h_of[0]
+                red = StructuredEngine(one, [self.f_pp_np[np.ix_(P0, P0)], self.f_ph_np[np.ix_(P0, H0)],
+                                             self.f_hh_np[np.ix_(H0, H0)]], self.dev, labels=m)
+                cat = lambda xs: torch.as_tensor(np.concatenate(xs).astype(np.int32), device=self.dev)  # noqa: E731
+                red.orders = cat(self.plan.p_of), cat(self.plan.h_of)
+                red.sizes = self.plan.p, self.plan.h
+                red.full_plan = self.plan
+            self.cache["reduced"] = red
+        red = self.cache["reduced"]
+        if red is not None:
+            red.tune = self.tune
+            if self._prob is not None:
+                for name in ("uniform_nh", "diag_ladders", "max_fpp_offdiag"):
+                    setattr(red.prob, name, getattr(self._prob, name))
+                for name in ("h_row", "fph_prow", "fpp_prow", "t1c_idx", "xc_ki"):
+                    setattr(red.prob, name, red.tables[name].data_ptr() if getattr(self._prob, name) else None)
+        return red
+
+    def expand_t1(self, t1):
+        """t1 of one label (this reduced engine's) -> the full [p, h] (device)."""
+        out = torch.empty(self.sizes, dtype=torch.float64, device=self.dev)
+        self._expand(t1, out, None, None, False)
+        return out
+
+    def expand_t2(self, t2, dense=False, out=None):
+        """The block of every pair -> the compact t2 of all pairs, or the dense one."""
+        p, h = self.sizes
+        if dense:
+            out = torch.zeros((p, p, h, h), dtype=torch.float64, device=self.dev)
+        elif out is None:
+            out = torch.empty(self.labels * (self.labels - 1) // 2 * self.plan.n_t2, dtype=t2.dtype, device=self.dev)
+        self._expand(None, None, t2, out, dense)
+        return out
+
+    def _expand(self, t1, t1_full, t2, t2_full, dense):
+        ptr = lambda x: None if x is None else x.data_ptr()  # noqa: E731
+        code = _lib.NLB_F32 if t2 is not None and t2.dtype == torch.float32 else _lib.NLB_F64
+        _lib.check(_lib.lib().nlb_sym_expand(self.prob, self.orders[0].data_ptr(), self.orders[1].data_ptr(), ptr(t1),
+                                             ptr(t1_full), ptr(t2), code, ptr(t2_full), int(dense),
+                                             _stream_ptr(self.dev)), "expand")
+        self.launches += 1
+
+    def compress(self, t1_full, t2_full):
+        """t1 of one label when amplitudes of the full layout (device, t2
+        compact) have the alike-label form -- labels bit for bit, exchange
+        to rounding -- else None.  The first block of ``t2_full`` is then t2."""
+        t1 = torch.empty(self.plan.p * self.plan.h, dtype=torch.float64, device=self.dev)
+        out = torch.empty(3, dtype=torch.int64, device=self.dev)
+        f32 = t2_full.dtype == torch.float32
+        _lib.check(_lib.lib().nlb_sym_check(self.prob, self.orders[0].data_ptr(), self.orders[1].data_ptr(),
+                                            t1_full.data_ptr(), t2_full.data_ptr(),
+                                            _lib.NLB_F32 if f32 else _lib.NLB_F64, t1.data_ptr(), out.data_ptr(),
+                                            _stream_ptr(self.dev)), "check")
+        self.launches += 1
+        o = out.cpu().numpy()
+        bad, (asym, big) = int(o[0]), o[1:].view(np.float64)
+        return t1 if bad == 0 and asym <= (1e-5 if f32 else 1e-8) * big else None
+
+    def _build(self):
+        pl = self.plan
+        f_pp, f_ph, f_hh = self.f_pp_np, self.f_ph_np, self.f_hh_np
+        device = self.dev
         G = pl.n_labels
         dev = device
         i32 = lambda a: torch.as_tensor(np.ascontiguousarray(a, dtype=np.int32), device=dev)  # noqa: E731
@@ -121,10 +237,9 @@ class StructuredEngine:
         n_p = np.array([len(x) for x in pl.p_of]); n_h = np.array([len(x) for x in pl.h_of])
         t1c_base = np.concatenate([[0], np.cumsum(n_p * n_h)]).astype(np.int32)
         xc_base = np.concatenate([[0], np.cumsum(n_h * n_h)]).astype(np.int32)
-        self.n_f2, self.n_rows, self.max_row = foff, rows, max_row
+        self.max_row = max_row
         self.max_nh = int(max(1, n_h.max() if len(n_h) else 1))
         self.n_t1c, self.n_xc = int(t1c_base[-1]), int(xc_base[-1])
-        self.n_g = goff
         cat = lambda xs, dt: np.concatenate(xs).astype(dt) if xs else np.zeros(1, dt)  # noqa: E731
         T = {}
         T["chan"] = torch.as_tensor(chans.view(np.uint8), device=dev)
@@ -160,7 +275,7 @@ class StructuredEngine:
             xc_ki.append((H_[:, None] * pl.h + H_[None, :]).ravel())
         T["t1c_idx"] = i32(cat(t1c_idx, np.int64))
         T["xc_ki"] = i32(cat(xc_ki, np.int64))
-        self.tables = T
+        self._tables = T
         prob = _lib.StructProblem()
         prob.p, prob.h, prob.n_labels, prob.n_channels = pl.p, pl.h, G, len(pl.channels)
         prob.n_t2, prob.n_g, prob.n_f2, prob.n_rows = pl.n_t2, self.n_g, self.n_f2, self.n_rows
@@ -192,10 +307,8 @@ class StructuredEngine:
         prob.max_fpp_offdiag = int(np.bincount(row_id[offd], minlength=1).max()) if offd.any() else 0
         for k, v in T.items():
             setattr(prob, k, v.data_ptr())
-        self.prob = prob
-        self._bufs = {}
-        self.cache = {}
-        self.launches = 0
+        prob.tune = self._tune_word()
+        self._prob = prob
 
     # -- buffers ---------------------------------------------------------
     def buffers(self, dtype_code, max_diis):
@@ -481,7 +594,7 @@ def ccsd_solver(fock_mats, two_body_int, t1initial=None, eps=1e-8, maxSteps=1000
         t0 = time.perf_counter()
         eng = StructuredEngine(plan, fock_mats, dev)
         from . import tune as _tune
-        eng.prob.tune = _tune.known_word(eng)   # cached or default launch shapes, no timing
+        eng.tune = _tune.known_word(eng)   # cached or default launch shapes, no timing
         info["t_engine"] = time.perf_counter() - t0
         t0 = time.perf_counter()
         e, t1, t2 = solve_structured(eng, t1initial=t1initial, eps=eps, maxSteps=maxSteps,
@@ -516,19 +629,30 @@ def solve_structured(eng, t1initial=None, eps=1e-8, maxSteps=1000, max_diis=10, 
     the host, which costs no graph build and suits an engine used once."""
     info = {} if info is None else info
     L = _lib.lib()
-    pl, dev = eng.plan, eng.dev
+    full, red = eng, eng.reduced()
     crit = _CRIT[criterion]
-    if t1initial is None:
+    t1_start = None
+    if t1initial is not None:
+        t1_start = np.asarray(_np(t1initial), dtype=np.float64)
+        if red is not None:   # one label only when the start has the form
+            blocks = [t1_start[np.ix_(P, H)] for P, H in zip(full.plan.p_of, full.plan.h_of)]
+            alike = all(np.array_equal(blocks[0], x) for x in blocks[1:]) and \
+                np.count_nonzero(t1_start) == len(blocks) * np.count_nonzero(blocks[0])
+            red, t1_start = (red, blocks[0]) if alike else (None, t1_start)
+    eng = full if red is None else red
+    launches0 = eng.launches
+    pl, dev = eng.plan, eng.dev
+    if t1_start is None:
         # MP2 start, computed once per engine and delta and kept on the device
         key = ("mp2", float(delta))
         if key not in eng.cache:
             t1 = _mp2_t1(eng.f_pp_np, eng.f_ph_np, eng.f_hh_np, float(delta))
-            eng.cache[key] = (torch.as_tensor(np.ascontiguousarray(t1), device=dev), float(np.sum(eng.f_ph_np * t1)))
+            eng.cache[key] = (torch.as_tensor(np.ascontiguousarray(t1), device=dev),
+                              eng.labels * float(np.sum(eng.f_ph_np * t1)))
         t1_dev, e0 = eng.cache[key]
     else:
-        t1 = np.asarray(_np(t1initial), dtype=np.float64)
-        e0 = float(np.sum(eng.f_ph_np * t1))
-        t1_dev = torch.as_tensor(np.ascontiguousarray(t1), device=dev)
+        e0 = eng.labels * float(np.sum(eng.f_ph_np * t1_start))
+        t1_dev = torch.as_tensor(np.ascontiguousarray(t1_start), device=dev)
     diis = int(max_diis) if crit == _lib.NLB_CRIT_SOA else 0
     sp = ctypes_void(torch.cuda.current_stream(dev).cuda_stream)
     iters = 0
@@ -591,12 +715,18 @@ def solve_structured(eng, t1initial=None, eps=1e-8, maxSteps=1000, max_diis=10, 
     info["t_iterate"] = time.perf_counter() - t0
     info["status"] = _STATUS[c.status]
     info["iterations"] = iters
-    info["n_t2"] = pl.n_t2
-    info["plan"] = pl.info
+    info["n_t2"] = full.plan.n_t2
+    info["n_t2_stored"] = pl.n_t2
+    info["plan"] = full.plan.info
     cur = c.parity
     e = float(c.e_last)
-    t1_out = b["t1"][cur].reshape(pl.p, pl.h).clone()
     dcode = b["state"].dtype
+    if red is not None:
+        t1_out = red.expand_t1(b["t1"][cur])
+        t2_out = red.expand_t2(b["t2"][cur], dense=t2_format != "compact")
+        full.launches += red.launches - launches0
+        return e, t1_out, t2_out
+    t1_out = b["t1"][cur].reshape(pl.p, pl.h).clone()
     if t2_format == "compact":
         t2_out = b["t2"][cur][:pl.n_t2].clone()
     else:

@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) k_t2_rows(nlb_struct_problem P
         __syncthreads();
     }
     const double s = block_sum(nrm);
-    if (threadIdx.x == 0) V.slots(kRedDt2)[blockIdx.x] = 4.0 * s;
+    if (threadIdx.x == 0) V.slots(kRedDt2)[blockIdx.x] = t2_weight(P) * s;
 }
 
 // ------------------------------------------------ T2 update, lattice path ----
@@ -733,7 +733,7 @@ __global__ void __launch_bounds__(NT, MINB) k_t2_lat(nlb_struct_problem P, nlb_s
         mis = next_mis;
     }
     const double s = block_sum(nrm);
-    if (threadIdx.x == 0) V.slots(kRedDt2)[blockIdx.x] = 4.0 * s;
+    if (threadIdx.x == 0) V.slots(kRedDt2)[blockIdx.x] = t2_weight(P) * s;
 }
 
 #include "t2_pair.cuh"
@@ -760,6 +760,7 @@ __global__ void __launch_bounds__(kThreads) k_t1_update(nlb_struct_problem P, nl
     double* E1 = (S.diis_t1 != nullptr && c->max_diis > 0 && c->diis_count < c->max_diis)
                      ? S.diis_t1 + (int64_t)c->diis_count * p * h : nullptr;
     const double m = c->mixing;
+    const double others = sym_others(P);   // alike labels: the channels of a label are copies of the stored one
     double eacc = 0.0, nrm = 0.0;
     const int64_t n = (int64_t)p * h;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -818,7 +819,7 @@ __global__ void __launch_bounds__(kThreads) k_t1_update(nlb_struct_problem P, nl
                     }
                 }
 #pragma unroll
-                for (int u = 0; u < 4; ++u) part += cp[u];
+                for (int u = 0; u < 4; ++u) part += others * cp[u];
                 // holes of a channel beyond the sixteen lanes
                 for (int u = 0; u < 4 && c0 + u < P.n_channels; ++u) {
                     const nlb_channel& ch = P.chan[c0 + u];
@@ -858,8 +859,8 @@ __global__ void __launch_bounds__(kThreads) k_t1_update(nlb_struct_problem P, nl
     const double se = block_sum(eacc);
     const double sn = block_sum(nrm);
     if (threadIdx.x == 0) {
-        V.slots(kRedE)[blockIdx.x] = se;
-        V.slots(kRedDt1)[blockIdx.x] = sn;
+        V.slots(kRedE)[blockIdx.x] = sym_labels(P) * se;
+        V.slots(kRedDt1)[blockIdx.x] = sym_labels(P) * sn;
     }
 }
 
@@ -927,7 +928,10 @@ __global__ void __launch_bounds__(kThreads) k_diis_gram(nlb_struct_problem P, nl
     nlb_ctrl* c = S.ctrl;
     if (!c->diis_pulse) return;
     constexpr int NP = M * (M + 1) / 2;
-    A acc[NP];   // sum of w/4 * e_s e_t: T1 entries weigh 1/4 here, T2 entries 1
+    // sum of e_s e_t / w with T2 entries weighing 1 (w dense entries each) and
+    // T1 entries m / w (m alike labels; 1/4 when every label is stored)
+    A acc[NP];
+    const double w2 = t2_weight(P), w1 = sqrt(sym_labels(P) / w2);
 #pragma unroll
     for (int k = 0; k < NP; ++k) acc[k] = A(0);
     const int64_t n1 = (int64_t)P.p * P.h;
@@ -937,14 +941,14 @@ __global__ void __launch_bounds__(kThreads) k_diis_gram(nlb_struct_problem P, nl
     for (int64_t e = tid0; e < n1; e += stride) {
         A v[M];
 #pragma unroll
-        for (int s = 0; s < M; ++s) v[s] = (A)(0.5 * S.diis_t1[(int64_t)s * n1 + e]);
+        for (int s = 0; s < M; ++s) v[s] = (A)(w1 * S.diis_t1[(int64_t)s * n1 + e]);
         int k = 0;
 #pragma unroll
         for (int s = 0; s < M; ++s)
 #pragma unroll
             for (int t = s; t < M; ++t) acc[k++] += v[s] * v[t];
     }
-    // T2 part, weight 4 (four images per stored amplitude)
+    // T2 part
     const T* E2 = static_cast<const T*>(S.diis_t2);
     for (int64_t e = tid0; e < n2; e += 2 * stride) {
         const int64_t e2 = e + stride;
@@ -969,7 +973,7 @@ __global__ void __launch_bounds__(kThreads) k_diis_gram(nlb_struct_problem P, nl
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
-        const double v = warp_sum(4.0 * (double)acc[k]);
+        const double v = warp_sum(w2 * (double)acc[k]);
         if (lane == 0) red[wid][k] = v;
     }
     __syncthreads();
@@ -1152,7 +1156,7 @@ __global__ void __launch_bounds__(1024) k_energy(nlb_struct_problem P, nlb_struc
     double acc = 0.0;
     for (int64_t e = threadIdx.x; e < n; e += blockDim.x) acc += P.f_ph[e] * t1[e];
     const double s = block_sum(acc);
-    if (threadIdx.x == 0) *out = s;
+    if (threadIdx.x == 0) *out = sym_labels(P) * s;
 }
 
 __global__ void k_ctrl_init(nlb_ctrl* c, double eps, double mixing, int max_steps, int criterion,
@@ -1287,6 +1291,8 @@ bool use_lat(const nlb_struct_problem* P, size_t el) {
 int valid(const nlb_struct_problem* P, const nlb_struct_state* S) {
     if (!P || !S || !S->ctrl) return fail(NLB_ERR_ARG, "null problem/state");
     if (P->p <= 0 || P->h <= 0 || P->n_channels < 0) return fail(NLB_ERR_SIZE, "bad p/h/channels");
+    if (sym_labels(*P) > 1 && (P->n_labels != 1 || P->n_channels != 1))
+        return fail(NLB_ERR_ARG, "alike labels: one stored label with one channel");
     if (S->dtype != NLB_F64 && S->dtype != NLB_F32) return fail(NLB_ERR_ARG, "dtype must be NLB_F64 or NLB_F32");
     if (!S->t1[0] || !S->t1[1] || !S->prep) return fail(NLB_ERR_ARG, "null t1/prep buffer");
     if (P->n_t2 > 0 && (!S->t2[0] || !S->t2[1] || !S->g || !S->f2)) return fail(NLB_ERR_ARG, "null t2/g/f2 buffer");

@@ -30,6 +30,27 @@ __device__ double block_sum(double v) {
     return v;  // valid in thread 0
 }
 
+// ----------------------------------------------------- alike labels ----
+// A label-symmetric problem stores one label and its one channel (0, 0) for m
+// labels that are all alike (bits 24-31 of the tuning word): t1 counts m times,
+// t2 once per pair of labels, and a label meets m - 1 others.  m = 1: every
+// label is stored.
+__host__ __device__ inline int sym_labels(const nlb_struct_problem& P) {
+    const int m = (int)((uint32_t)P.tune >> 24);
+    return m > 1 ? m : 1;
+}
+__host__ __device__ inline double sym_pairs(const nlb_struct_problem& P) {
+    const int m = sym_labels(P);
+    return m > 1 ? 0.5 * m * (m - 1) : 1.0;
+}
+// channels of a label beyond the stored one's share: m - 1 (all stored: 1)
+__host__ __device__ inline double sym_others(const nlb_struct_problem& P) {
+    const int m = sym_labels(P);
+    return m > 1 ? (double)(m - 1) : 1.0;
+}
+// dense entries of one stored t2 amplitude: four antisymmetric images per pair
+__device__ __forceinline__ double t2_weight(const nlb_struct_problem& P) { return 4.0 * sym_pairs(P); }
+
 // ---------------------------------------------------------------- prep ----
 // Layout of the prep scratch (doubles), see nlb_struct_prep_len:
 //   Q[h*h]   Q[k,j] = sum_c f_ck t1_cj

@@ -305,8 +305,8 @@ __global__ void __launch_bounds__(kThreads) k_l_rows(nlb_struct_problem P, nlb_l
     const double s1 = block_sum(dnrm);
     const double s2 = block_sum(lnrm);
     if (tid == 0) {
-        PV.slots(kRedDt2)[blockIdx.x] = 4.0 * s1;
-        PV.slots(kRedNrm2)[blockIdx.x] = 4.0 * s2;
+        PV.slots(kRedDt2)[blockIdx.x] = t2_weight(P) * s1;
+        PV.slots(kRedNrm2)[blockIdx.x] = t2_weight(P) * s2;
     }
 }
 
@@ -343,6 +343,12 @@ __global__ void k_l_u(nlb_struct_problem P, nlb_lambda_state S) {
     }
 }
 
+// Alike labels: the stored channel (0, 0) gives a label both its sides, each of
+// which stands for half of the label's m - 1 channels.
+__device__ __forceinline__ double sym_half(const nlb_struct_problem& P) {
+    return sym_labels(P) > 1 ? 0.5 * sym_others(P) : 1.0;
+}
+
 // General path: Y1 and T from the row kernel's slots.  Thread per entry of
 // Y1 (p*h) or T (h*h); the channels in order, the rows of a channel in order.
 __global__ void k_l_rows_reduce(nlb_struct_problem P, nlb_lambda_state S) {
@@ -350,6 +356,7 @@ __global__ void k_l_rows_reduce(nlb_struct_problem P, nlb_lambda_state S) {
     if (c->status != NLB_RUNNING) return;
     const LView V = lview(S.acc, P);
     const int h = P.h, mh = P.max_nh;
+    const double half = sym_half(P);
     const int64_t ph = (int64_t)P.p * h, hh = (int64_t)h * h;
     for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < ph + hh;
          idx += (int64_t)gridDim.x * blockDim.x) {
@@ -367,7 +374,7 @@ __global__ void k_l_rows_reduce(nlb_struct_problem P, nlb_lambda_state S) {
                             y += V.Yg[ch.offset + ((int64_t)ap * ch.np2 + xl) * ch.nh2 + ml];
                 }
             }
-            V.Y1[idx] = y;
+            V.Y1[idx] = half * y;
         } else {
             const int64_t u = idx - ph;
             const int k = (int)(u / h), mm = (int)(u % h);
@@ -385,7 +392,7 @@ __global__ void k_l_rows_reduce(nlb_struct_problem P, nlb_lambda_state S) {
                     }
                 }
             }
-            V.T[u] = t;
+            V.T[u] = half * t;
         }
     }
 }
@@ -425,6 +432,7 @@ __global__ void k_l_t1(nlb_struct_problem P, nlb_lambda_state S, int nchunk) {
                 if (ch.g2 == g)
                     for (int cq = 0; cq < nchunk; ++cq) y1 += V.Y1c[(int64_t)cq * P.n_f2 + o];
             }
+            y1 *= sym_half(P);
         } else {
             y1 = V.Y1[idx];
         }
@@ -451,8 +459,8 @@ __global__ void k_l_t1(nlb_struct_problem P, nlb_lambda_state S, int nchunk) {
     const double s1 = block_sum(dn);
     const double s2 = block_sum(ln);
     if (threadIdx.x == 0) {
-        PV.slots(kRedDt1)[blockIdx.x] = s1;
-        PV.slots(kRedNrm1)[blockIdx.x] = s2;
+        PV.slots(kRedDt1)[blockIdx.x] = sym_labels(P) * s1;
+        PV.slots(kRedNrm1)[blockIdx.x] = sym_labels(P) * s2;
     }
 }
 
@@ -546,7 +554,7 @@ __global__ void k_l_coupling(nlb_struct_problem P, nlb_lambda_state S, const dou
         }
     }
     const double s = block_sum(acc);
-    if (threadIdx.x == 0) PV.slots(0)[blockIdx.x] = s;
+    if (threadIdx.x == 0) PV.slots(0)[blockIdx.x] = sym_pairs(P) * s;
 }
 
 // *out = the n per-block partials at `part`, added in slot order (one warp).
@@ -795,7 +803,7 @@ __global__ void k_l_treduce(nlb_struct_problem P, nlb_lambda_state S, int nchunk
         s = block_sum(s);
         if (threadIdx.x == 0) {
             const int hb = P.h_base[g];
-            V.T[(int64_t)P.h_ord[hb + w / kLH] * P.h + P.h_ord[hb + w % kLH]] = s;
+            V.T[(int64_t)P.h_ord[hb + w / kLH] * P.h + P.h_ord[hb + w % kLH]] = sym_half(P) * s;
         }
         return;
     }
@@ -1111,8 +1119,8 @@ __global__ void __launch_bounds__(NT, MINB) k_l_lat(nlb_struct_problem P, nlb_la
     const double s1 = block_sum(dnrm);
     const double s2 = block_sum(lnrm);
     if (tid == 0) {
-        PV.slots(kRedDt2)[blockIdx.x] = 4.0 * s1;
-        PV.slots(kRedNrm2)[blockIdx.x] = 4.0 * s2;
+        PV.slots(kRedDt2)[blockIdx.x] = t2_weight(P) * s1;
+        PV.slots(kRedNrm2)[blockIdx.x] = t2_weight(P) * s2;
     }
 }
 

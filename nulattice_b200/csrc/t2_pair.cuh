@@ -370,5 +370,5 @@ __global__ void __launch_bounds__(NT, MINB) k_t2_pair(nlb_struct_problem P, nlb_
         blo = 0;
     }
     const double s = block_sum(nrm);
-    if (threadIdx.x == 0) V.slots(kRedDt2)[blockIdx.x] = 4.0 * s;
+    if (threadIdx.x == 0) V.slots(kRedDt2)[blockIdx.x] = t2_weight(P) * s;
 }

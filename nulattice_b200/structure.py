@@ -334,3 +334,58 @@ def detect(fock_mats, two_body_int, t1initial=None):
                      dense_t2=p * p * h * h, fpp_nnz=len(fpp_val), fph_nnz=len(fph_val),
                      pp_nnz=int(sum(len(x) for x in pp_val)), hh_nnz=int(sum(len(x) for x in hh_val)))
     return plan, None
+
+
+def alike_labels(plan, f_hh):
+    """``(label plan, m)`` when all m labels of ``plan`` are alike, else None.
+
+    Labels are alike when they have the same f_pp, f_ph and f_hh blocks and
+    every pair of them the same ladders, symmetric under exchange of the two
+    labels.  Then all labels have the same t1 and all pairs the same t2 (from
+    a start that has), and one label with one channel (0, 0) describes the
+    problem: every lattice nucleus of closed sites with an SU(4) contact.
+    """
+    m, chs = plan.n_labels, plan.channels
+    if m < 2 or m > 255 or len(chs) != m * (m - 1) // 2:
+        return None
+    n, h = len(plan.p_of[0]), len(plan.h_of[0])
+    if n == 0 or h == 0 or any(len(x) != n for x in plan.p_of) or any(len(x) != h for x in plan.h_of):
+        return None
+
+    def same_csr(ptr, col, val, rows):
+        """Equal runs of ``rows`` CSR rows per label."""
+        ptr = np.asarray(ptr)
+        per = int(ptr[rows])
+        return (int(ptr[-1]) == m * per and
+                np.array_equal(np.diff(ptr).reshape(m, rows), np.tile(np.diff(ptr[:rows + 1]), (m, 1))) and
+                np.array_equal(np.reshape(col, (m, per)), np.tile(col[:per], (m, 1))) and
+                np.array_equal(np.reshape(val, (m, per)), np.tile(val[:per], (m, 1))))
+
+    if not same_csr(plan.fpp_ptr, plan.fpp_col, plan.fpp_val, n) or \
+            not same_csr(plan.fph_ptr, plan.fph_col, plan.fph_val, h):
+        return None
+    f_hh = np.asarray(f_hh)
+    f0 = f_hh[np.ix_(plan.h_of[0], plan.h_of[0])]
+    if any(not np.array_equal(f_hh[np.ix_(x, x)], f0) for x in plan.h_of):
+        return None
+    for ptr, col, val, k in ((plan.hh_ptr, plan.hh_col, plan.hh_val, h), (plan.pp_ptr, plan.pp_col, plan.pp_val, n)):
+        if any(not (np.array_equal(ptr[0], a) and np.array_equal(col[0], b) and np.array_equal(val[0], c))
+               for a, b, c in zip(ptr[1:], col[1:], val[1:])):
+            return None
+        # exchange of the two labels: pair x1 * k + x2 -> x2 * k + x1 on both sides
+        out = np.repeat(np.arange(k * k), np.diff(ptr[0]))
+        swap = lambda x: (x % k) * k + x // k  # noqa: E731
+        key, key2 = out * (k * k) + col[0], swap(out) * (k * k) + swap(np.asarray(col[0]))
+        o1, o2 = np.argsort(key, kind="stable"), np.argsort(key2, kind="stable")
+        if not (np.array_equal(key[o1], key2[o2]) and np.array_equal(val[0][o1], val[0][o2])):
+            return None
+    zn, zh = np.zeros(n, np.int64), np.zeros(h, np.int64)
+    npp, nph = int(plan.fpp_ptr[n]), int(plan.fph_ptr[h])
+    one = ChannelPlan(p=n, h=h, n_labels=1, p_label=zn, h_label=zh, p_loc=np.arange(n), h_loc=np.arange(h),
+                      p_of=[np.arange(n)], h_of=[np.arange(h)], channels=[Channel(0, 0, n, n, h, h, 0)],
+                      n_t2=n * n * h * h, p_base=np.array([0, n]), h_base=np.array([0, h]),
+                      fpp_ptr=plan.fpp_ptr[:n + 1], fpp_col=plan.fpp_col[:npp], fpp_val=plan.fpp_val[:npp],
+                      fph_ptr=plan.fph_ptr[:h + 1], fph_col=plan.fph_col[:nph], fph_val=plan.fph_val[:nph],
+                      hh_ptr=plan.hh_ptr[:1], hh_col=plan.hh_col[:1], hh_val=plan.hh_val[:1],
+                      pp_ptr=plan.pp_ptr[:1], pp_col=plan.pp_col[:1], pp_val=plan.pp_val[:1])
+    return one, m

@@ -37,7 +37,7 @@ def known_word(eng):
     on B200 at L=6, A=28 (two-row T2 kernel with 384 threads, Lambda column
     pass in two row chunks).  Non-lattice problems: 0 (no choices)."""
     L = _lib.lib()
-    if not L.nlb_lambda_lattice(eng.prob):
+    if not L.nlb_lambda_lattice((eng.reduced() or eng).prob):
         return 0
     path = _cache_path()
     if os.path.exists(path):
@@ -72,9 +72,11 @@ def _cache_path():
 
 
 def _key(eng):
-    pl, prob = eng.plan, eng.prob
+    work = eng.reduced() or eng
+    pl, nh = work.plan, work.prob.uniform_nh
     name = torch.cuda.get_device_name(eng.dev)
-    return f"{name}|p={pl.p}|h={pl.h}|n_t2={pl.n_t2}|nh={prob.uniform_nh}|ch={prob.n_channels}"
+    alike = f"|alike={work.labels}" if work.labels > 1 else ""
+    return f"{name}|p={pl.p}|h={pl.h}|n_t2={pl.n_t2}|nh={nh}|ch={len(pl.channels)}{alike}"
 
 
 def _time(fn, reps):
@@ -96,10 +98,11 @@ def tune(eng, lam=True, reps=7, use_cache=True, info=None):
     the defaults.  Returns the tuning word."""
     L = _lib.lib()
     info = {} if info is None else info
+    full, eng = eng, eng.reduced() or eng     # the shapes are timed on the problem that runs
     if not L.nlb_lambda_lattice(eng.prob):
-        eng.prob.tune = 0
+        full.tune = 0
         return 0
-    key = _key(eng)
+    key = _key(full)
     path = _cache_path()
     cache = {}
     if use_cache and os.path.exists(path):
@@ -108,9 +111,9 @@ def tune(eng, lam=True, reps=7, use_cache=True, info=None):
         except (OSError, ValueError):
             cache = {}
     if use_cache and key in cache:
-        eng.prob.tune = int(cache[key]["word"])
+        full.tune = int(cache[key]["word"])
         info.update(cache[key], cached=True)
-        return eng.prob.tune
+        return full.tune
     dev = eng.dev
     sp = ctypes_void(torch.cuda.current_stream(dev).cuda_stream)
     pl = eng.plan
@@ -128,7 +131,7 @@ def tune(eng, lam=True, reps=7, use_cache=True, info=None):
             _lib.check(L.nlb_struct_step(eng.prob, b["state"], sp), "step")
         res = {}
         for v in variants:
-            eng.prob.tune = v << shift
+            eng.tune = v << shift
 
             def run():
                 _lib.check(L.nlb_struct_stage(eng.prob, b["state"], _lib.NLB_STAGE_T2, sp), "stage")
@@ -148,7 +151,7 @@ def tune(eng, lam=True, reps=7, use_cache=True, info=None):
         res = {}
         for lv in LAM_F32:
             for c in cands:
-                eng.prob.tune = word(lam32=lv, chunks=c)
+                eng.tune = word(lam32=lv, chunks=c)
                 _lib.check(L.nlb_lambda_init(eng.prob, b["state"], 0.0, 0.5, 1 << 30, 0, 0, sp), "lambda_init")
 
                 def run():
@@ -158,7 +161,7 @@ def tune(eng, lam=True, reps=7, use_cache=True, info=None):
         lam32, chunks = min(res, key=res.get)
         times["lambda_fp32"] = {f"{LAM_F32[lv]}/chunks={c or 'auto'}": round(t * 1e3, 1) for (lv, c), t in res.items()}
     w = word(fwd32=best["t2_fp32"], lam32=lam32, chunks=chunks, fwd64=best["t2_fp64"])
-    eng.prob.tune = w
+    full.tune = eng.tune = w
     entry = {"word": w, "choice": describe(w), "us": times}
     info.update(entry, cached=False)
     if use_cache:

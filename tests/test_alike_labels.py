@@ -1,0 +1,152 @@
+"""Label-symmetric problems: one label and one channel stand for all of them.
+
+On the CPU the conditions under which the labels count as alike; on the GPU
+every path that then runs on one label (solves, Lambda steps, gradients)
+against the same path with every label stored."""
+import numpy as np
+import pytest
+import torch
+
+from nulattice_b200 import _lib
+from nulattice_b200 import adjoint as A
+from nulattice_b200 import hamiltonian as ham
+from nulattice_b200 import structure as S
+from nulattice_b200.ccsd import StructuredEngine, solve_structured
+
+SEVEN = [(0, 0, 0), (1, 0, 0), (-1, 0, 0), (0, 1, 0), (0, -1, 0), (0, 0, 1), (0, 0, -1)]
+
+
+def _inputs(L, sites, C2=-3.1, C3=0.9):
+    holes = [[x % L, y % L, z % L, t, s] for (x, y, z) in SEVEN[:sites] for t in (0, 1) for s in (0, 1)]
+    v, w = ham.contact_couplings(C2, C3)
+    _, fock, two = ham.normal_ordered_hamiltonian(L, holes, v, v, w, dense=False)
+    return holes, [f.copy() for f in fock], two
+
+
+@pytest.mark.parametrize("L,sites", [(3, 1), (3, 2), (4, 7)])
+def test_lattice_labels_are_alike(L, sites):
+    _, fock, two = _inputs(L, sites)
+    plan, _ = S.detect(fock, two)
+    one, m = S.alike_labels(plan, fock[2])
+    assert m == 4 and one.n_labels == 1 and len(one.channels) == 1
+    assert (one.p, one.h, one.n_t2) == (plan.p // 4, plan.h // 4, plan.n_t2 // 6)
+
+
+@pytest.mark.parametrize("what", ["f_pp", "f_ph", "f_hh", "pp", "hh", "exchange"])
+def test_labels_that_differ_are_not_alike(what):
+    _, fock, two = _inputs(3, 2)
+    plan, _ = S.detect(fock, two)
+    P, H = plan.p_of[1], plan.h_of[1]
+    if what == "f_pp":
+        fock[0][P[3], P[3]] += 1e-9
+    elif what == "f_ph":
+        i, j = np.argwhere(fock[1][np.ix_(P, H)])[0]
+        fock[1][P[i], H[j]] *= 1.5
+    elif what == "f_hh":
+        fock[2][H[0], H[0]] += 0.25
+    plan, _ = S.detect(fock, two)
+    if what == "pp":
+        plan.pp_val[2] = plan.pp_val[2] * 2
+    elif what == "hh":
+        plan.hh_val[5] = plan.hh_val[5] + 1
+    elif what == "exchange":   # the same in every channel, but not under exchange of the labels
+        for n in range(6):
+            plan.pp_ptr[n] = np.concatenate([[0, 0], np.ones(plan.channels[n].np1 ** 2 - 1, np.int64)])
+            plan.pp_col[n], plan.pp_val[n] = np.array([1]), np.array([1.0])   # pair (0, 1) only
+    assert S.alike_labels(plan, fock[2]) is None
+
+
+def _engine(L, sites, full=False):
+    holes, fock, two = _inputs(L, sites)
+    plan, _ = S.detect(fock, two)
+    eng = StructuredEngine(plan, fock, torch.device("cuda:0"))
+    if full:
+        eng.cache["reduced"] = None
+    assert (eng.reduced() is None) == full
+    return holes, eng
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,sites", [(3, 1), (3, 2), (4, 3), (3, 7), (4, 7), (5, 7)])
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-13), ("mixed", 4e-7)])
+def test_solve_on_one_label(L, sites, precision, tol):
+    """Six steps before a DIIS pulse (rounding only), both layouts of t2, then
+    a pulsed FP64 solve to convergence."""
+    out = {}
+    for full in (False, True):
+        _, eng = _engine(L, sites, full)
+        for fmt in ("compact", "dense") if L == 3 else ("compact",):
+            for loop in ("graph", "eager"):
+                info = {}
+                e, t1, t2 = solve_structured(eng, eps=0.0, mixed_eps=0.0, maxSteps=6, max_diis=8, refine=False,
+                                             precision=precision, t2_format=fmt, loop=loop, info=info)
+                out[full, fmt, loop] = e, t1.cpu().numpy(), t2.double().cpu().numpy()
+                assert info["n_t2_stored"] == (eng.plan.n_t2 if full else eng.plan.n_t2 // 6)
+        info = {}
+        e, t1, t2 = solve_structured(eng, eps=1e-12, maxSteps=400, max_diis=8, t2_format="compact", info=info)
+        assert info["status"] == "converged"
+        out[full, "converged"] = e, t1.cpu().numpy(), t2.cpu().numpy()
+    for key in out:
+        if key[0]:
+            continue
+        lim = 1e-7 if key[1] == "converged" else tol
+        for got, want in zip(out[key], out[(True,) + key[1:]]):
+            assert np.abs(np.asarray(got) - want).max() <= lim * np.abs(want).max(), key
+
+
+@pytest.mark.gpu
+def test_a_start_that_treats_labels_differently_runs_on_all():
+    _, eng = _engine(3, 7)
+    t1 = np.zeros((eng.plan.p, eng.plan.h))
+    P, H = eng.plan.p_of[2], eng.plan.h_of[2]
+    t1[P[0], H[0]] = 1e-3
+    out = []
+    for full in (False, True):
+        _, eng = _engine(3, 7, full)
+        info = {}
+        out.append(solve_structured(eng, t1initial=t1, eps=0.0, maxSteps=4, max_diis=8, t2_format="compact", info=info))
+        assert info["n_t2_stored"] == eng.plan.n_t2
+    assert out[0][0] == out[1][0] and torch.equal(out[0][2], out[1][2])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,sites,code,tol", [(3, 1, _lib.NLB_F64, 1e-12), (3, 3, _lib.NLB_F64, 1e-12),
+                                              (4, 7, _lib.NLB_F64, 1e-12), (4, 7, _lib.NLB_F32, 2e-6)])
+def test_lambda_steps_on_one_label(L, sites, code, tol):
+    """Lambda steps (from zero, then kept), U and T included; amplitudes that
+    treat one pair of labels differently run with every label stored."""
+    got = {}
+    for full in (False, True):
+        _, eng = _engine(L, sites, full)
+        _, t1, t2 = solve_structured(eng, eps=1e-13, max_diis=8, maxSteps=2000, t2_format="compact")
+        if not full:
+            start = t1, t2
+        solver = A.LambdaSolver(eng)
+        b = solver.buffers(code, 0)
+        b["t1"].copy_(start[0].reshape(-1))
+        b["t2"].copy_(start[1])
+        c = solver.run(b, 0.0, 0.5, 3, 0, False)
+        ph, hh = eng.plan.p * eng.plan.h, eng.plan.h ** 2
+        b["lam1"][0].copy_(b["lam1"][c.parity].clone())
+        b["lam2"][0].copy_(b["lam2"][c.parity].clone())
+        c = solver.run(b, 0.0, 0.5, 3, 0, True)
+        assert (solver._label is None) == full
+        got[full] = [x.double().cpu().numpy() for x in (b["lam1"][c.parity], b["lam2"][c.parity],
+                                                        b["acc"][ph:ph + 2 * hh])]
+        if not full:
+            b["t2"][-1] += 0.5
+            assert solver._alike(b, False) is None
+    for x, y in zip(got[False], got[True]):
+        assert np.abs(x - y).max() <= tol * np.abs(y).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,sites,precision", [(3, 1, "fp64"), (3, 7, "mixed")])
+def test_gradient_on_one_label(L, sites, precision):
+    grads = []
+    for full in (False, True):
+        holes, eng = _engine(L, sites, full)
+        prob = A.lattice_problem(L, holes)
+        _, t1, t2 = solve_structured(eng, eps=1e-13, max_diis=8, maxSteps=2000, t2_format="compact")
+        grads.append(A.lambda_gradient(eng, t1, t2, [prob.dv, prob.dw], tol=1e-10, precision=precision))
+    np.testing.assert_allclose(grads[0], grads[1], rtol=1e-8)
