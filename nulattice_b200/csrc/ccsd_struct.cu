@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(kThreads) k_prep_ga(nlb_struct_problem P, nlb_
     const int64_t nga_blocks = (c->ccs || P.n_t2 == 0) ? 0 : (int64_t)P.n_channels * P.max_nh * gx;
     const int64_t all_ga = (int64_t)P.n_channels * P.max_nh * gx;
     if ((int64_t)blockIdx.x >= all_ga) {
-        const double* t1 = S.t1[c->parity];
+        const double* t1 = t1_buf(S, c->parity);
         const int64_t nb = gridDim.x - all_ga;
         for (int64_t u = ((int64_t)blockIdx.x - all_ga) * blockDim.x + threadIdx.x; u < nprep; u += nb * blockDim.x)
             prep_body(P, t1, S.prep, u);
@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(kThreads) k_prep_ga(nlb_struct_problem P, nlb_
     const int rowlen = ch.np2 * ch.nh1 * ch.nh2;
     const int row = ch.hb1 + kq;
     const int q0 = P.fph_ptr[row], q1 = P.fph_ptr[row + 1];
-    const T* __restrict__ Bc = static_cast<const T*>(S.t2[c->parity]) + ch.offset;
+    const T* __restrict__ Bc = t2_buf<const T>(S, c->parity) + ch.offset;
     // Ga layout per channel: [b'][k'][i'j'] (the k' values of one (b', i'j')
     // one hole-pair stride apart, so a reader needs one address per b')
     const int nhp = ch.nh1 * ch.nh2;
@@ -741,18 +741,18 @@ __global__ void __launch_bounds__(NT, MINB) k_t2_lat(nlb_struct_problem P, nlb_s
 // --------------------------------------------------------- T1 update ----
 // R1 = f_ph + F2 + f_pp t1 - t1 Q/2 + t1 X_hh(T1 eq); Jacobi + mixing;
 // energy sum_ai f_ai t1'_ai (coupled_cluster.py:342-414, 265-286).
+// Block bid of nblk (the T1 partial sums go to slot bid).
 template <typename T>
-__global__ void __launch_bounds__(kThreads) k_t1_update(nlb_struct_problem P, nlb_struct_state S) {
+__device__ void t1_body(const nlb_struct_problem& P, const nlb_struct_state& S, int bid, int nblk) {
     // Sixteen lanes per amplitude t1[a, i] of matching labels (the others
     // are zero for label-conserving inputs and stay zero); the lanes share
     // the terms of its residual: the T2 Fock terms of the channels holding
     // the label (F2, or the Ga diagonal), the f_pp neighbours of a and the
     // hole mixing over the label's holes.
-    nlb_ctrl* c = S.ctrl;
-    if (c->status != NLB_RUNNING) return;
+    const nlb_ctrl* c = S.ctrl;
     const int par = c->parity;
-    const double* t1 = S.t1[par];
-    double* t1o = S.t1[par ^ 1];
+    const double* t1 = t1_buf(S, par);
+    double* t1o = t1_buf(S, par ^ 1);
     const int h = P.h, p = P.p;
     const PrepView V = prep_view(S.prep, P);
     const T* Ga = static_cast<const T*>(S.g);
@@ -763,8 +763,8 @@ __global__ void __launch_bounds__(kThreads) k_t1_update(nlb_struct_problem P, nl
     const double others = sym_others(P);   // alike labels: the channels of a label are copies of the stored one
     double eacc = 0.0, nrm = 0.0;
     const int64_t n = (int64_t)p * h;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += stride) {
+    const int64_t stride = (int64_t)nblk * blockDim.x;
+    for (int64_t idx = (int64_t)bid * blockDim.x + threadIdx.x; idx < n; idx += stride) {
         const int a = (int)(idx / h), i = (int)(idx - (int64_t)a * h);
         if (P.h_label[i] != P.p_label[a]) {
             t1o[idx] = 0.0;
@@ -775,7 +775,7 @@ __global__ void __launch_bounds__(kThreads) k_t1_update(nlb_struct_problem P, nl
     // its residual is an independent load, so one wave covers all of them
     const int lane = threadIdx.x & 15;
     const int64_t nhalf = stride >> 4;
-    for (int64_t q0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
+    for (int64_t q0 = ((int64_t)bid * blockDim.x + threadIdx.x) >> 4;
          q0 - (((int64_t)threadIdx.x >> 4) & 1) < P.n_t1c; q0 += nhalf) {
         // both halves of a warp stay in the loop until neither has work
         const bool live = q0 < P.n_t1c;
@@ -859,27 +859,41 @@ __global__ void __launch_bounds__(kThreads) k_t1_update(nlb_struct_problem P, nl
     const double se = block_sum(eacc);
     const double sn = block_sum(nrm);
     if (threadIdx.x == 0) {
-        V.slots(kRedE)[blockIdx.x] = sym_labels(P) * se;
-        V.slots(kRedDt1)[blockIdx.x] = sym_labels(P) * sn;
+        V.slots(kRedE)[bid] = sym_labels(P) * se;
+        V.slots(kRedDt1)[bid] = sym_labels(P) * sn;
     }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kThreads) k_t1_update(nlb_struct_problem P, nlb_struct_state S) {
+    if (S.ctrl->status != NLB_RUNNING) return;
+    t1_body<T>(P, S, blockIdx.x, gridDim.x);
 }
 
 // -------------------------------------------------- convergence test ----
 // One warp: the step's energy and norms from the per-block partials of the
 // T1 (n1 blocks) and T2 (n2 blocks) launches, added in slot order.
-// Launched with three warps: warp w adds one partial-sum array (energy, T1
-// step, T2 step), each in the fixed order of warp_sum_slots.
-__global__ void k_finish(nlb_ctrl* c, const double* red, int n1, int n2) {
-    __shared__ double sums[3];
-    if (blockIdx.x != 0) return;
-    if (c->status != NLB_RUNNING) return;
-    const int w = threadIdx.x >> 5;
-    if (w == 0) sums[0] = warp_sum_slots(red + (int64_t)kRedE * kRedSlots, n1);
-    else if (w == 1) sums[1] = warp_sum_slots(red + (int64_t)kRedDt1 * kRedSlots, n1);
-    else if (w == 2) sums[2] = c->ccs ? 0.0 : warp_sum_slots(red + (int64_t)kRedDt2 * kRedSlots, n2);
+// The warps share the T2 step partials (one per block of its launch, up to a
+// few thousand) in contiguous runs; the first two also add the energy and the
+// T1 step.  Every run is in the fixed order of warp_sum_slots.
+constexpr int kFinishThreads = 256;
+
+__device__ void finish_body(nlb_ctrl* c, const double* red, int n1, int n2) {
+    __shared__ double sums[2 + 32];
+    const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int q = c->ccs ? 0 : n2;
+    const int b0 = (int)((int64_t)w * q / nw), b1 = (int)((int64_t)(w + 1) * q / nw);
+    double v = warp_sum_slots(red + (int64_t)kRedDt2 * kRedSlots + b0, b1 - b0);
+    if ((threadIdx.x & 31) == 0) sums[2 + w] = v;
+    for (int k = w; k < 2; k += nw) {
+        v = warp_sum_slots(red + (int64_t)(k == 0 ? kRedE : kRedDt1) * kRedSlots, n1);
+        if ((threadIdx.x & 31) == 0) sums[k] = v;
+    }
     __syncthreads();
     if (threadIdx.x != 0) return;
-    const double e_sum = sums[0], d1 = sums[1], d2 = sums[2];
+    const double e_sum = sums[0], d1 = sums[1];
+    double d2 = 0.0;
+    for (int k = 0; k < nw; ++k) d2 += sums[2 + k];
     c->e_acc = e_sum;
     c->dt1_sq = d1;
     c->dt2_sq = d2;
@@ -911,6 +925,12 @@ __global__ void k_finish(nlb_ctrl* c, const double* red, int n1, int n2) {
     c->e_prev = E;
 }
 
+__global__ void __launch_bounds__(kFinishThreads) k_finish(nlb_ctrl* c, const double* red, int n1, int n2) {
+    if (c->status != NLB_RUNNING) return;
+    finish_body(c, red, n1, n2);
+}
+
+#include "t2_sym.cuh"
 
 // ---------------------------------------------------------------- DIIS ----
 // Gram matrix of the stored error vectors: <e_a, e_b> over the dense t1 and
@@ -919,12 +939,12 @@ constexpr int kMaxDiis = 10;
 
 template <typename T, int M>
 __global__ void __launch_bounds__(kThreads) k_diis_gram(nlb_struct_problem P, nlb_struct_state S) {
-    // FP32 error vectors: products and per-thread partial sums in FP32 (the
-    // sums cover a few hundred elements, relative error ~1e-5, well inside
-    // what the extrapolation needs), block and grid sums in FP64; FP64
-    // vectors: FP64 throughout.  Two elements per thread and step keep
-    // 2M loads in flight.
-    using A = T;
+    // Products and sums in FP64 for either vector type: the vectors are nearly
+    // parallel, and an FP32 sum's 1e-6 costs the extrapolation digits (40
+    // couplings each at A=4 and 28, L=3-5, mixed solves to 1e-12: 25-30
+    // iterations on average against 28-33 with FP32 sums).  Two elements per
+    // thread and step keep 2M loads in flight.
+    using A = double;
     nlb_ctrl* c = S.ctrl;
     if (!c->diis_pulse) return;
     constexpr int NP = M * (M + 1) / 2;
@@ -964,7 +984,7 @@ __global__ void __launch_bounds__(kThreads) k_diis_gram(nlb_struct_problem P, nl
         for (int s = 0; s < M; ++s)
 #pragma unroll
             for (int t = s; t < M; ++t) {
-                acc[k] += v[s] * v[t] + u[s] * u[t];
+                acc[k] += (A)v[s] * (A)v[t] + (A)u[s] * (A)u[t];
                 ++k;
             }
     }
@@ -1372,10 +1392,98 @@ int64_t t1_grid(const nlb_struct_problem* P) {
     return reducing_grid(blocks_per_sm(reinterpret_cast<const void*>(k_t1_update<T>), 0), need);
 }
 
+// The two-launch step of a label-symmetric problem (t2_sym.cuh): diagonal
+// ladders, f_pp rows of at most kSymNf entries, at most seven holes (a thread
+// keeps the sums of all hole pairs), a row in shared memory.
+// Columns of a block of the update pass: four loads of a thread at least;
+// twice and four times that while two blocks per SM are left (a block's fixed
+// cost, the chain of its first loads and its count, is 2-3 us; A=28 L=6, 1199
+// -> 390 blocks: 17.2 -> 16.4 us FP32, 27.1 -> 20.5 us FP64).
+template <int NH>
+int sym_cols(int p) {
+    int cols = 4 * (kThreads / (NH * NH));
+    for (int k = 0; k < 2 && sym_blocks(p, 2 * cols) >= 2 * num_sms(); ++k) cols *= 2;
+    return cols;
+}
+
+template <typename T, int NH>
+bool sym_fits(const nlb_struct_problem* P) {
+    return sym_smem<T, NH>(P->p, kSymMost).total + 2048 <= smem_limit() &&
+           sym_blocks(P->p, sym_cols<NH>(P->p)) <= 2 * kRedSlots;
+}
+
+// Calls f.template operator()<NH>() for the problem's hole count.
+template <typename F>
+auto sym_holes(int h, F f) {
+    switch (h) {
+        case 1: return f.template operator()<1>();
+        case 2: return f.template operator()<2>();
+        case 3: return f.template operator()<3>();
+        case 4: return f.template operator()<4>();
+        case 5: return f.template operator()<5>();
+        case 6: return f.template operator()<6>();
+        default: return f.template operator()<7>();
+    }
+}
+
+template <typename T>
+struct SymFits {
+    const nlb_struct_problem* P;
+    template <int NH> bool operator()() const { return sym_fits<T, NH>(P); }
+};
+
+template <typename T>
+bool use_sym(const nlb_struct_problem* P) {
+    return sym_labels(*P) > 1 && P->n_t2 > 0 && P->diag_ladders == 1 && P->max_fpp_offdiag <= kSymNf && P->h >= 1 &&
+           P->h <= 7 && P->max_nh == P->h && P->p <= kRedSlots && sym_holes(P->h, SymFits<T>{P});
+}
+
+template <typename T>
+struct SymRow {
+    const nlb_struct_problem* P;
+    const nlb_struct_state* S;
+    cudaStream_t st;
+    template <int NH> int operator()() const {
+        auto kern = k_sym_row<T, NH>;
+        // runs of columns per row: two blocks per SM, whole warps
+        constexpr int PARTS = sym_parts<T>(NH);
+        int runs = (2 * num_sms() + P->p - 1) / P->p;
+        const int most = (P->p + 31) / 32, least = (P->p + kSymMost - 1) / kSymMost;
+        runs = runs > most ? most : runs;
+        runs = runs < least ? least : runs;
+        int nc = ((P->p + runs - 1) / runs + 31) / 32 * 32;
+        nc = nc * PARTS < 128 ? (128 / PARTS + 31) / 32 * 32 : nc;   // the staging and the tables want threads, too
+        const int nt = nc * PARTS;
+        const int64_t sm = sym_smem<T, NH>(P->p, nc).total;
+        blocks_per_sm(reinterpret_cast<const void*>(kern), sm, nt);   // raises the shared-memory limit
+        kern<<<(unsigned)(P->p * runs), nt, (size_t)sm, st>>>(*P, *S, runs);
+        return 0;
+    }
+};
+
+template <typename T>
+struct SymUpdate {
+    const nlb_struct_problem* P;
+    const nlb_struct_state* S;
+    int fin;
+    cudaStream_t st;
+    bool launch;
+    template <int NH> int64_t operator()() const {
+        const int cols = sym_cols<NH>(P->p);
+        const int64_t n2 = sym_blocks(P->p, cols);
+        if (launch) k_sym_update<T, NH><<<(unsigned)n2, kThreads, 0, st>>>(*P, *S, cols, fin);
+        return n2;
+    }
+};
+
 template <typename T>
 void stage_t(const nlb_struct_problem* P, const nlb_struct_state* S, int stage, cudaStream_t st) {
     switch (stage) {
         case NLB_STAGE_PREP: {
+            if (use_sym<T>(P)) {   // the row sums of the T2 residual, and T1
+                sym_holes(P->h, SymRow<T>{P, S, st});
+                break;
+            }
             const int64_t nprep = (int64_t)P->h * P->h + 2 * (int64_t)P->p + P->n_t1c + P->n_xc + P->h;
             // the dressed-Fock tables and Ga in one launch (the GTERMS stage is then empty)
             const int64_t per_blk = (int64_t)kThreads * kGaVec;
@@ -1389,20 +1497,28 @@ void stage_t(const nlb_struct_problem* P, const nlb_struct_state* S, int stage, 
         case NLB_STAGE_GTERMS:
             break;   // Ga is formed with the prep tables
         case NLB_STAGE_T2:
-            t2_update<T>(P, S, st, true);
+            if (use_sym<T>(P)) sym_holes(P->h, SymUpdate<T>{P, S, 0, st, true});
+            else t2_update<T>(P, S, st, true);
             break;
         case NLB_STAGE_T1:
+            if (use_sym<T>(P)) break;   // with the row sums
             k_t1_update<T><<<(unsigned)t1_grid<T>(P), kThreads, 0, st>>>(*P, *S);
             break;
         default:
-            k_finish<<<1, 96, 0, st>>>(S->ctrl, prep_view(S->prep, *P).red, (int)t1_grid<T>(P),
-                                       (int)t2_update<T>(P, S, st, false));
+            k_finish<<<1, kFinishThreads, 0, st>>>(
+                S->ctrl, prep_view(S->prep, *P).red, use_sym<T>(P) ? P->p : (int)t1_grid<T>(P),
+                (int)(use_sym<T>(P) ? sym_holes(P->h, SymUpdate<T>{P, S, 0, st, false}) : t2_update<T>(P, S, st, false)));
     }
 }
 
 template <typename T>
 int step_t(const nlb_struct_problem* P, const nlb_struct_state* S, cudaStream_t st) {
-    for (int k = NLB_STAGE_PREP; k <= NLB_STAGE_FINISH; ++k) stage_t<T>(P, S, k, st);
+    if (use_sym<T>(P)) {
+        sym_holes(P->h, SymRow<T>{P, S, st});
+        sym_holes(P->h, SymUpdate<T>{P, S, 1, st, true});   // with the convergence test
+    } else {
+        for (int k = NLB_STAGE_PREP; k <= NLB_STAGE_FINISH; ++k) stage_t<T>(P, S, k, st);
+    }
     return check_launch("nlb_struct_step");
 }
 

@@ -104,7 +104,7 @@ __host__ __device__ inline PrepView prep_view(double* base, const nlb_struct_pro
 // with the same n; all lanes return the same value.
 __device__ __forceinline__ double warp_sum_slots(const double* part, int n) {
     double s = 0.0;
-    for (int b = (int)(threadIdx.x & 31); b < n; b += 32) s += part[b];
+    for (int b = (int)(threadIdx.x & 31); b < n; b += 32) s += __ldcg(part + b);
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     return s;
 }
@@ -252,6 +252,13 @@ __device__ __forceinline__ T ga_element(const nlb_struct_problem& P, const T* B,
     return acc;
 }
 
+// The amplitude buffer of parity par (a selection: indexing the parameter's
+// array with a run-time value would copy the whole struct to local memory).
+template <typename T, typename S>
+__device__ __forceinline__ T* t2_buf(const S& s, int par) { return static_cast<T*>(par ? s.t2[1] : s.t2[0]); }
+template <typename S>
+__device__ __forceinline__ double* t1_buf(const S& s, int par) { return par ? s.t1[1] : s.t1[0]; }
+
 __host__ __device__ inline int64_t lat_round16(int64_t b) { return (b + 15) & ~int64_t(15); }
 
 // Work units of channel cc for the row kernels that split rows by b'
@@ -295,6 +302,16 @@ __device__ __forceinline__ void lds8(const int32_t* p, int (&v)[8]) {
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
+
+// Four consecutive shared-memory values (16-byte aligned) with vector loads.
+__device__ __forceinline__ void lds4(const float* p, float (&v)[4]) {
+    const float4 a = *reinterpret_cast<const float4*>(p);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+__device__ __forceinline__ void lds4(const double* p, double (&v)[4]) {
+    const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
 
 // Jacobi quotient R / D.  FP32 amplitudes: the approximate reciprocal (the
 // denominators only set the step length, the fixed point R = 0 does not

@@ -95,6 +95,24 @@ def test_solve_on_one_label(L, sites, precision, tol):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("L,sites", [(2, 1), (3, 4), (3, 5), (3, 6), (4, 6), (5, 1), (7, 1)])
+@pytest.mark.parametrize("precision,eps", [("fp64", 2.0 ** -53), ("mixed", 2.0 ** -24)])
+def test_step_kernels_over_hole_counts_and_row_lengths(L, sites, precision, eps):
+    """Three steps on one label (row and pair kernels) against every label stored
+    (general kernels): rows shorter than a warp up to longer than a block, every
+    hole count.  A step's sum has at most 14 + 4 h + 2 roundings of terms no
+    larger than the result's norm; eight for their ratio to the largest element."""
+    out = {}
+    for full in (False, True):
+        _, eng = _engine(L, sites, full)
+        e, t1, t2 = solve_structured(eng, eps=0.0, mixed_eps=0.0, maxSteps=3, max_diis=0, refine=False,
+                                     precision=precision, t2_format="compact")
+        out[full] = e, t1.cpu().numpy(), t2.double().cpu().numpy()
+    for got, want in zip(out[False], out[True]):
+        assert np.abs(np.asarray(got) - want).max() <= 3 * 8 * (16 + 4 * sites) * eps * np.abs(want).max()
+
+
+@pytest.mark.gpu
 def test_a_start_that_treats_labels_differently_runs_on_all():
     _, eng = _engine(3, 7)
     t1 = np.zeros((eng.plan.p, eng.plan.h))
