@@ -340,27 +340,16 @@ __global__ void k_pw_R(nlb_pw_problem P, const F* __restrict__ t2, F* __restrict
     }
 }
 
-template <typename F>
-__device__ __forceinline__ F dot16(const F* __restrict__ x, const F* __restrict__ y) {
-    F s = 0;
-    if constexpr (sizeof(F) == 8) {
+__device__ __forceinline__ float dot16(const float* __restrict__ x, const float* __restrict__ y) {
+    float s = 0;
 #pragma unroll
-        for (int q = 0; q < 16; q += 2) {
-            const double2 a = *reinterpret_cast<const double2*>(x + q);
-            const double2 c = *reinterpret_cast<const double2*>(y + q);
-            s += a.x * c.x;
-            s += a.y * c.y;
-        }
-    } else {
-#pragma unroll
-        for (int q = 0; q < 16; q += 4) {
-            const float4 a = *reinterpret_cast<const float4*>(x + q);
-            const float4 c = *reinterpret_cast<const float4*>(y + q);
-            s += a.x * c.x;
-            s += a.y * c.y;
-            s += a.z * c.z;
-            s += a.w * c.w;
-        }
+    for (int q = 0; q < 16; q += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(x + q);
+        const float4 c = *reinterpret_cast<const float4*>(y + q);
+        s += a.x * c.x;
+        s += a.y * c.y;
+        s += a.z * c.z;
+        s += a.w * c.w;
     }
     return s;
 }
@@ -373,7 +362,32 @@ __device__ __forceinline__ F dot16(const F* __restrict__ x, const F* __restrict_
 // row and column groups sit in shared memory.  The quadratic ring term uses
 // Z(ai, bj) = R_ai V R_bj = Z(bj, ai) (V[c d k l] = V[d c l k]), so its four
 // images reduce to 2 (Z(ai, bj) - Z(bi, aj)).
+//
+// FP64: both contractions run on the double-precision tensor instruction, warp
+// w taking rows 8 w .. 8 w + 7 of the tile.  Z of a row group and the column
+// group is the 16 x 16 product of U and R over 16 spin pairs, so the warp reads
+// each of their vectors once, as fragments straight from global memory (a
+// thread's four k are neighbours: the order of a sum over k is free).  One dot
+// product per amplitude read 512 bytes for each and kept the load unit busy 90%
+// of 181 us (A=28 L=6, 2.5 M amplitudes); 88.7 us this way.
 constexpr int kTR = 64, kTC = 16;
+
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+        : "+d"(d[0]), "+d"(d[1])
+        : "d"(a), "d"(b));
+}
+
+// Eight vectors of 16 starting at X (four of one row of `ld` vectors, four of
+// the next) as a fragment: lane (g, k4) holds elements 4 k4 .. 4 k4 + 3 of vector g.
+__device__ __forceinline__ void frag16(const double* __restrict__ X, int64_t ld, int g, int k4, double (&f)[4]) {
+    const double2* p = reinterpret_cast<const double2*>(X + ((g >> 2) * ld + (g & 3)) * 16 + 4 * k4);
+    const double2 x = p[0], y = p[1];
+    f[0] = x.x;
+    f[1] = x.y;
+    f[2] = y.x;
+    f[3] = y.y;
+}
 
 template <typename F>
 __global__ void __launch_bounds__(256) k_pw_residual(nlb_pw_problem P, const F* __restrict__ t2,
@@ -381,9 +395,12 @@ __global__ void __launch_bounds__(256) k_pw_residual(nlb_pw_problem P, const F* 
                                                      const F* __restrict__ Xpp, const F* __restrict__ Xhh,
                                                      const F* __restrict__ R, const F* __restrict__ U,
                                                      const F* __restrict__ G, F* __restrict__ H) {
-    __shared__ F Ts[kTR][kTC + 1];
+    constexpr bool TC = sizeof(F) == 8;
+    constexpr int PAD = TC ? 4 : 1;   // a stride of 20 doubles: fragments without bank conflicts
+    __shared__ F Ts[kTR][kTC + PAD];
     __shared__ F Town[kTR][kTC + 1];
-    __shared__ F Ws[kTC][kTC + 1];
+    __shared__ F Ws[kTC][kTC + PAD];
+    __shared__ F Zs[TC ? kTR : 1][kTC + 1];   // T_K W_K + the quadratic ring term
     __shared__ F Vs[256];
     __shared__ int s_ma[4], s_mb[4], s_mi, s_mj;
     const int tid = threadIdx.x;
@@ -411,6 +428,42 @@ __global__ void __launch_bounds__(256) k_pw_residual(nlb_pw_problem P, const F* 
         }
         const F* T = t2 + P.blk_off[b];
         const F* Wb = W + P.w_off[b];
+        const int w8 = (tid >> 5) * 8, g = (tid >> 2) & 7, k4 = tid & 3;   // fragment coordinates
+        if constexpr (TC) {
+            __syncthreads();
+            const int q = w8 >> 4, h2 = (w8 >> 3) & 1;   // row group; its rows s_a = 2 h2, 2 h2 + 1 are the warp's
+            const int64_t i = s_mi * 4, j = s_mj * 4, a = s_ma[q] * 4 + 2 * h2, bb = s_mb[q] * 4;
+            double u[4], v[4], z[2][2];
+            // U_ai R_bj: rows (s_a, s_i), columns (s_b, s_j)
+            frag16(U + (a * nhs + i) * 16, nhs, g, k4, u);
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                frag16(R + ((bb + 2 * n) * nhs + j) * 16, nhs, g, k4, v);
+                z[n][0] = z[n][1] = 0.0;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) dmma(z[n], u[k], v[k]);
+            }
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+                    Zs[w8 + (g >> 2) * 4 + 2 * n + (k4 >> 1)][(g & 3) * 4 + (k4 & 1) * 2 + e] = z[n][e];
+            // U_bi R_aj: rows (s_b, s_i), columns (s_a, s_j)
+            frag16(R + (a * nhs + j) * 16, nhs, g, k4, v);
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                frag16(U + ((bb + 2 * n) * nhs + i) * 16, nhs, g, k4, u);
+                z[n][0] = z[n][1] = 0.0;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) dmma(z[n], u[k], v[k]);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+                    Zs[w8 + (k4 >> 1) * 4 + 2 * n + (g >> 2)][(g & 3) * 4 + (k4 & 1) * 2 + e] -= z[n][e];
+        }
         F acc[4] = {0.0, 0.0, 0.0, 0.0};
         for (int k0 = 0; k0 < nc; k0 += kTC) {
             __syncthreads();
@@ -425,12 +478,33 @@ __global__ void __launch_bounds__(256) k_pw_residual(nlb_pw_problem P, const F* 
             }
             Ws[rr][cc] = Wb[(int64_t)(k0 + rr) * nc + c0 + cc];
             __syncthreads();
+            if constexpr (TC) {
+                double (&d)[4] = acc;
 #pragma unroll
-            for (int kk = 0; kk < kTC; ++kk) {
-                const F w = Ws[kk][cc];
+                for (int kk = 0; kk < kTC; kk += 4) {
+                    const double x = Ts[w8 + g][kk + k4];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) acc[q] += Ts[rr + 16 * q][kk] * w;
+                    for (int n = 0; n < 2; ++n)
+                        dmma(*reinterpret_cast<double (*)[2]>(&d[2 * n]), x, Ws[kk + k4][8 * n + g]);
+                }
+            } else {
+#pragma unroll
+                for (int kk = 0; kk < kTC; ++kk) {
+                    const F w = Ws[kk][cc];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) acc[q] += Ts[rr + 16 * q][kk] * w;
+                }
             }
+        }
+        if constexpr (TC) {
+            __syncwarp();
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) Zs[w8 + g][8 * n + 2 * k4 + e] += acc[2 * n + e];
+            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[q] = Zs[rr + 16 * q][cc];
         }
         const F* Mb = M + P.m_off[b];
         const int c = c0 + cc;
@@ -472,8 +546,8 @@ __global__ void __launch_bounds__(256) k_pw_residual(nlb_pw_problem P, const F* 
             const int64_t aj = (a * nhs + j) * 16, bj = (bb * nhs + j) * 16;
             const F ring = ((G[ai + sb * 4 + sj] - G[bi + sa * 4 + sj]) -
                                  (G[aj + sb * 4 + si] - G[bj + sa * 4 + si]));
-            const F quad = dot16(U + ai, R + bj) - dot16(U + bi, R + aj);
-            h += ring + quad;
+            h += ring;
+            if constexpr (!TC) h += dot16(U + ai, R + bj) - dot16(U + bi, R + aj);
             H[P.blk_off[b] + (int64_t)r * nc + c] = h;
         }
     }
