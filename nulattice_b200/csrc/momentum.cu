@@ -126,23 +126,36 @@ __global__ void k_pw_init(nlb_pw_problem P, double* t2, double delta) {
 }
 
 // ------------------------------------------------------------ M, energy ----
-// M_K[sigma][c] = sum_pa T_K[pa*16 + sigma][c]: one warp per entry, the
-// lanes over the row groups pa, summed by a fixed shuffle tree.
+// M_K[sigma][c] = sum_pa T_K[pa*16 + sigma][c].  A block forms 32 neighbouring
+// entries of one momentum block (their rows repeat every 16 nc amplitudes, so a
+// warp reads 32 neighbours of one pa), its warps over the row groups pa; the
+// eight partial sums are added in warp order.  A lane per pa read one amplitude
+// of every 32-byte sector: 19.5 us for A=28 L=6 FP64, 8.9 us this way.
+constexpr int kPwMEntries = 32;
+
 template <typename F>
-__global__ void k_pw_M(nlb_pw_problem P, const F* __restrict__ t2, F* __restrict__ M) {
-    const int lane = threadIdx.x & 31;
-    const int64_t wpb = blockDim.x >> 5;
-    for (int64_t e = (int64_t)blockIdx.x * wpb + (threadIdx.x >> 5); e < P.n_m; e += (int64_t)gridDim.x * wpb) {
-        const int b = seg_of(P.m_off, P.n_blocks, e);
-        const int nc = P.blk_nc[b];
-        const int64_t loc = e - P.m_off[b];
-        const int sg = (int)(loc / nc), c = (int)(loc % nc);
+__global__ void __launch_bounds__(256) k_pw_M(nlb_pw_problem P, const F* __restrict__ t2, F* __restrict__ M) {
+    __shared__ F part[8][kPwMEntries];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t n = P.n_m / kPwMEntries;   // 16 nc entries per block, nc a multiple of 16: no remainder
+    for (int64_t u = blockIdx.x; u < n; u += gridDim.x) {
+        const int64_t e = u * kPwMEntries + lane;
+        const int b = seg_of(P.m_off, P.n_blocks, u * kPwMEntries);
         const int npa = P.blk_nr[b] >> 4;
-        const F* T = t2 + P.blk_off[b] + (int64_t)sg * nc + c;
+        const int64_t step = (int64_t)16 * P.blk_nc[b];
+        const F* T = t2 + P.blk_off[b] + (e - P.m_off[b]);
         F acc = 0.0;
-        for (int pa = lane; pa < npa; pa += 32) acc += T[(int64_t)pa * 16 * nc];
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) M[e] = acc;
+#pragma unroll 4
+        for (int pa = w; pa < npa; pa += 8) acc += T[pa * step];
+        part[w][lane] = acc;
+        __syncthreads();
+        if (w == 0) {
+            F m = part[0][lane];
+#pragma unroll
+            for (int k = 1; k < 8; ++k) m += part[k][lane];
+            M[e] = m;
+        }
+        __syncthreads();
     }
 }
 
@@ -180,40 +193,42 @@ __global__ void k_pw_energy_sum(const double* __restrict__ part, int n, double* 
 }
 
 // ------------------------------------------------------------ X_pp rows ----
-// One warp per row (pa, s_b, s_d) of every block:
+// Rows (pa, s_b, s_d) of every block:
 //   Y[row][s_c] = sum_c V[s_c s_d][spins of c] T[row][c]
+// Sixteen lanes per row, one per spin pair of the columns: a lane adds its
+// column of every column group, multiplies by the four V and the lanes' four
+// sums are reduced together (halves exchanged: five shuffles instead of four
+// trees of them).  With 32 lanes over the columns and four trees: 30.5 us for
+// A=28 L=6 FP64, 14.6 us this way.
 template <typename F>
-__global__ void k_pw_xrow(nlb_pw_problem P, const F* __restrict__ t2, F* __restrict__ Y) {
+__global__ void __launch_bounds__(256) k_pw_xrow(nlb_pw_problem P, const F* __restrict__ t2, F* __restrict__ Y) {
     __shared__ F Vs[256];
     for (int q = threadIdx.x; q < 256; q += blockDim.x) Vs[q] = P.V[q];
     __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const int64_t nrows = P.n_rows;
-    const int64_t wpb = blockDim.x >> 5;
-    for (int64_t row = (int64_t)blockIdx.x * wpb + (threadIdx.x >> 5); row < nrows; row += (int64_t)gridDim.x * wpb) {
+    const int sp = threadIdx.x & 15;
+    const int64_t nrows = P.n_rows;      // a multiple of 16: both rows of a warp are live
+    const int64_t rpb = blockDim.x >> 4;
+    for (int64_t row = (int64_t)blockIdx.x * rpb + (threadIdx.x >> 4); row < nrows; row += (int64_t)gridDim.x * rpb) {
         const int b = seg_of(P.row_off, P.n_blocks, row);
         const int r = (int)(row - P.row_off[b]);
         const int nc = P.blk_nc[b];
         const int sd = r & 3;
-        const F* T = t2 + P.blk_off[b] + (int64_t)r * nc;
-        F a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-        for (int c = lane; c < nc; c += 32) {
-            const F x = T[c];
-            const int sp = c & 15;
-            a0 += Vs[(0 * 4 + sd) * 16 + sp] * x;
-            a1 += Vs[(1 * 4 + sd) * 16 + sp] * x;
-            a2 += Vs[(2 * 4 + sd) * 16 + sp] * x;
-            a3 += Vs[(3 * 4 + sd) * 16 + sp] * x;
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-            a1 += __shfl_xor_sync(0xffffffffu, a1, o);
-            a2 += __shfl_xor_sync(0xffffffffu, a2, o);
-            a3 += __shfl_xor_sync(0xffffffffu, a3, o);
-        }
-        if (lane == 0) {
-            Y[row * 4 + 0] = a0; Y[row * 4 + 1] = a1; Y[row * 4 + 2] = a2; Y[row * 4 + 3] = a3;
-        }
+        const F* T = t2 + P.blk_off[b] + (int64_t)r * nc + sp;
+        F x = 0.0;
+#pragma unroll 4
+        for (int c = 0; c < nc; c += 16) x += T[c];
+        F a[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) a[q] = Vs[(q * 4 + sd) * 16 + sp] * x;
+        // lanes with bit 3 set keep s_c = 2, 3, then bit 2 the odd one
+        const bool h3 = sp & 8, h2 = sp & 4;
+        F y0 = __shfl_xor_sync(0xffffffffu, h3 ? a[0] : a[2], 8), y1 = __shfl_xor_sync(0xffffffffu, h3 ? a[1] : a[3], 8);
+        y0 += h3 ? a[2] : a[0];
+        y1 += h3 ? a[3] : a[1];
+        F y = __shfl_xor_sync(0xffffffffu, h2 ? y0 : y1, 4) + (h2 ? y1 : y0);
+        y += __shfl_xor_sync(0xffffffffu, y, 2);
+        y += __shfl_xor_sync(0xffffffffu, y, 1);
+        if ((sp & 3) == 0) Y[row * 4 + (sp >> 2)] = y;
     }
 }
 
@@ -285,58 +300,62 @@ __global__ void k_pw_W(nlb_pw_problem P, const F* __restrict__ M, F* __restrict_
 }
 
 // ------------------------------------------------------- ring intermediates ----
-// One thread per (a, i) = (particle momentum, s_a) x (hole momentum, s_i):
+// (a, i) = (particle momentum, s_a) x (hole momentum, s_i):
 //   R[s_c s_k] = sum_{k_k} t2[a, (k_k + k_i - k_a, s_c), i, (k_k, s_k)]
 //   G[s_b s_j] = - sum V[s_b s_k s_c s_j] R[s_c s_k]        (dgram_bkcj_acik, ccDgrams.py:253-264)
 //   U[s_d s_l] = sum V[s_c s_d s_k s_l] R[s_c s_k]          (dgram_cdkl_acik_dblj, ccDgrams.py:279-290)
+// Sixteen lanes per (a, i), one per result: sixteen holes k_k at a time, a lane
+// finds the amplitudes of one of them and every lane then adds its (s_c, s_k) of
+// each; G and U take R from the other lanes.  One thread per (a, i) left the SMs
+// with 0.6 blocks each: 24.5 us for A=28 L=6 FP64, 22.5 us this way (A=4 L=5 FP32: 11.5 and 4.9).
 template <typename F>
-__global__ void k_pw_R(nlb_pw_problem P, const F* __restrict__ t2, F* __restrict__ R,
-                       F* __restrict__ U, F* __restrict__ G) {
+__global__ void __launch_bounds__(256) k_pw_R(nlb_pw_problem P, const F* __restrict__ t2, F* __restrict__ R,
+                                              F* __restrict__ U, F* __restrict__ G) {
     __shared__ F Vs[256];
     for (int q = threadIdx.x; q < 256; q += blockDim.x) Vs[q] = P.V[q];
     __syncthreads();
     const int L = P.L, L3 = L * L * L;
     const int nps = 4 * P.n_pmom, nhs = 4 * P.n_hmom;
-    const int64_t n = (int64_t)nps * nhs;
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t n = (int64_t)nps * nhs;        // a multiple of 16: both halves of a warp are live
+    const int l = threadIdx.x & 15, hi = l >> 2, lo = l & 3;
+    for (int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 4; e < n;
+         e += ((int64_t)gridDim.x * blockDim.x) >> 4) {
         const int al = (int)(e / nhs), il = (int)(e % nhs);
         const int ma = al >> 2, sa = al & 3, mi = il >> 2, si = il & 3;
         const int ka = P.pmom[ma], ki = P.hmom[mi];
-        F r[16];
-#pragma unroll
-        for (int q = 0; q < 16; ++q) r[q] = 0.0;
-        for (int mk = 0; mk < P.n_hmom; ++mk) {
-            const int kk = P.hmom[mk];
-            const int kc = msub(madd(kk, ki, L), ka, L);
-            if (P.pinv[kc] < 0) continue;
-            const int b = P.kblk[madd(ka, kc, L)];
-            const int pa = P.ppos[(int64_t)b * L3 + ka];
-            const int pi = P.hpos[(int64_t)b * L3 + ki];
-            const int nc = P.blk_nc[b];
-            const F* T = t2 + P.blk_off[b] + (int64_t)(pa * 16 + sa * 4) * nc + pi * 16 + si * 4;
-#pragma unroll
-            for (int sc = 0; sc < 4; ++sc)
-#pragma unroll
-                for (int sk = 0; sk < 4; ++sk) r[sc * 4 + sk] += T[(int64_t)sc * nc + sk];
-        }
-        F* Ro = R + e * 16;
-        F* Uo = U + e * 16;
-        F* Go = G + e * 16;
-#pragma unroll
-        for (int q = 0; q < 16; ++q) Ro[q] = r[q];
-        for (int x = 0; x < 4; ++x)
-            for (int y = 0; y < 4; ++y) {
-                F g = 0.0, u = 0.0;
-#pragma unroll
-                for (int sc = 0; sc < 4; ++sc)
-#pragma unroll
-                    for (int sk = 0; sk < 4; ++sk) {
-                        g += Vs[((x * 4 + sk) * 4 + sc) * 4 + y] * r[sc * 4 + sk];
-                        u += Vs[((sc * 4 + x) * 4 + sk) * 4 + y] * r[sc * 4 + sk];
-                    }
-                Go[x * 4 + y] = -g;
-                Uo[x * 4 + y] = u;
+        F r = 0.0;
+        for (int m0 = 0; m0 < P.n_hmom; m0 += 16) {
+            long long off = -1;   // of hole m0 + l: its first amplitude
+            int nc = 0;
+            if (m0 + l < P.n_hmom) {
+                const int kc = msub(madd(P.hmom[m0 + l], ki, L), ka, L);
+                if (P.pinv[kc] >= 0) {
+                    const int b = P.kblk[madd(ka, kc, L)];
+                    nc = P.blk_nc[b];
+                    off = P.blk_off[b] + (int64_t)(P.ppos[(int64_t)b * L3 + ka] * 16 + sa * 4) * nc +
+                          P.hpos[(int64_t)b * L3 + ki] * 16 + si * 4;
+                }
             }
+            const int cnt = min(16, P.n_hmom - m0);
+#pragma unroll 4
+            for (int k = 0; k < cnt; ++k) {
+                const long long o = __shfl_sync(0xffffffffu, off, k, 16);
+                const int w = __shfl_sync(0xffffffffu, nc, k, 16);
+                if (o >= 0) r += t2[o + (int64_t)hi * w + lo];
+            }
+        }
+        F g = 0.0, u = 0.0;
+#pragma unroll
+        for (int sc = 0; sc < 4; ++sc)
+#pragma unroll
+            for (int sk = 0; sk < 4; ++sk) {
+                const F x = __shfl_sync(0xffffffffu, r, sc * 4 + sk, 16);
+                g += Vs[((hi * 4 + sk) * 4 + sc) * 4 + lo] * x;
+                u += Vs[((sc * 4 + hi) * 4 + sk) * 4 + lo] * x;
+            }
+        R[e * 16 + l] = r;
+        G[e * 16 + l] = -g;
+        U[e * 16 + l] = u;
     }
 }
 
@@ -557,32 +576,60 @@ __global__ void __launch_bounds__(256) k_pw_residual(nlb_pw_problem P, const F* 
 // Exact antisymmetric projection over the orbit {abij, baij, abji, baji} (the
 // four images sit in the same block), Jacobi step with the dressed diagonal
 // denominators and mixing (coupled_cluster.py:538-545, 614-620).
+// One CTA per residual tile (four row groups x one column group): the momenta
+// and the positions of the exchanged rows and columns are those of the groups,
+// looked up once per tile; decoding every amplitude's made 71% of the issue
+// slots and 51.8 us of A=28 L=6 FP64, 25.0 us this way.
 template <typename F>
-__global__ void k_pw_jacobi(nlb_pw_problem P, const F* __restrict__ t2, const F* __restrict__ H,
-                            const F* __restrict__ Xpp, const F* __restrict__ Xhh, double mixing,
-                            F* __restrict__ out, F* __restrict__ err) {
-    // grid (chunks, momentum blocks): blockIdx.y is the block of t2
+__global__ void __launch_bounds__(256) k_pw_jacobi(nlb_pw_problem P, const F* __restrict__ t2, const F* __restrict__ H,
+                                                   const F* __restrict__ Xpp, const F* __restrict__ Xhh, double mixing,
+                                                   F* __restrict__ out, F* __restrict__ err) {
+    __shared__ int s_ma[4], s_mb[4], s_rb[4], s_mi, s_mj, s_cj;
+    const int tid = threadIdx.x, cc = tid & 15, rr = tid >> 4;
     const int L = P.L, L3 = L * L * L;
-    const int b = blockIdx.y;
-    const int64_t boff = P.blk_off[b], bn = P.blk_off[b + 1] - boff;
-    const int nc = P.blk_nc[b];
-    for (int64_t loc = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; loc < bn;
-         loc += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t e = boff + loc;
-        const Amp A = decode_amp(P, b, (int)(loc / nc), (int)(loc % nc));
-        const int rb = P.ppos[(int64_t)b * L3 + P.pmom[A.mb]] * 16 + A.sb * 4 + A.sa;
-        const int cj = P.hpos[(int64_t)b * L3 + P.hmom[A.mj]] * 16 + A.sj * 4 + A.si;
-        const F* Hb = H + A.off;
-        const F x_abij = Hb[loc], x_baij = Hb[(int64_t)rb * nc + A.c];
-        const F x_abji = Hb[(int64_t)A.r * nc + cj], x_baji = Hb[(int64_t)rb * nc + cj];
-        const F v = F(0.25) * ((x_abij - x_baij) - (x_abji - x_baji));
-        const F den = -((Xpp[A.ma * 16 + A.sa * 5] + Xpp[A.mb * 16 + A.sb * 5]) +
-                             (Xhh[A.mi * 16 + A.si * 5] + Xhh[A.mj * 16 + A.sj * 5]));
-        const F t = t2[e];
-        const F tn = t + v / den;
-        const F o = F(mixing) * t + F(1.0 - mixing) * tn;
-        out[e] = o;
-        if (err) err[e] = o - t;
+    const int si = cc >> 2, sj = cc & 3, sa = rr >> 2, sb = rr & 3;
+    for (int tile = blockIdx.x; tile < P.n_tiles; tile += gridDim.x) {
+        const int b = P.tiles[3 * tile], r0 = P.tiles[3 * tile + 1], c0 = P.tiles[3 * tile + 2];
+        const int nr = P.blk_nr[b], nc = P.blk_nc[b], K = P.blk_K[b];
+        __syncthreads();   // the previous tile is done with the shared tables
+        if (tid < 4) {
+            const int pa = (r0 >> 4) + tid;
+            int ma = 0, mb = 0, rb = 0;
+            if (pa * 16 < nr) {
+                ma = P.pm_list[P.blk_pm0[b] + pa];
+                const int kb = msub(K, P.pmom[ma], L);
+                mb = P.pinv[kb];
+                rb = P.ppos[(int64_t)b * L3 + kb] * 16;
+            }
+            s_ma[tid] = ma;
+            s_mb[tid] = mb;
+            s_rb[tid] = rb;
+        } else if (tid == 4) {
+            const int mi = P.hm_list[P.blk_hm0[b] + (c0 >> 4)];
+            const int kj = msub(K, P.hmom[mi], L);
+            s_mi = mi;
+            s_mj = P.hinv[kj];
+            s_cj = P.hpos[(int64_t)b * L3 + kj] * 16;
+        }
+        __syncthreads();
+        const int64_t off = P.blk_off[b];
+        const F* Hb = H + off;
+        const int c = c0 + cc, cj = s_cj + sj * 4 + si;
+        const F xh = Xhh[s_mi * 16 + si * 5] + Xhh[s_mj * 16 + sj * 5];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int r = r0 + rr + 16 * q;
+            if (r >= nr) continue;
+            const int64_t rb = s_rb[q] + sb * 4 + sa, e = off + (int64_t)r * nc + c;
+            const F v = F(0.25) * ((Hb[(int64_t)r * nc + c] - Hb[rb * nc + c]) -
+                                   (Hb[(int64_t)r * nc + cj] - Hb[rb * nc + cj]));
+            const F den = -((Xpp[s_ma[q] * 16 + sa * 5] + Xpp[s_mb[q] * 16 + sb * 5]) + xh);
+            const F t = t2[e];
+            const F tn = t + v / den;
+            const F o = F(mixing) * t + F(1.0 - mixing) * tn;
+            out[e] = o;
+            if (err) err[e] = o - t;
+        }
     }
 }
 
@@ -600,7 +647,7 @@ template <typename F>
 int pw_energy(const nlb_pw_problem* P, const F* t2, nlb_pw_state* S, cudaStream_t st, const char* name) {
     if (!pw_ok(P) || !t2 || !S || !S->M || !S->Y || !S->energy) return pfail(NLB_ERR_ARG, name);
     F* M = static_cast<F*>(S->M);
-    k_pw_M<F><<<pgrid(32 * P->n_m), 256, 0, st>>>(*P, t2, M);
+    k_pw_M<F><<<pgrid(P->n_m / kPwMEntries * 256), 256, 0, st>>>(*P, t2, M);
     // the FP64 partial sums go to S->Y (rebuilt from t2 by every step
     // before use): 4 * n_rows values of F hold 4 * n_rows * sizeof(F) / 8
     int64_t nparts = 4 * P->n_rows * (int64_t)sizeof(F) / 8;
@@ -620,22 +667,20 @@ int pw_step(const nlb_pw_problem* P, const F* t2, F* t2_out, F* err, double mixi
         !S->U || !S->G || !S->H)
         return pfail(NLB_ERR_ARG, name);
     if (P->n_blocks > 65535) return pfail(NLB_ERR_SIZE, "momentum step: more than 65535 momentum blocks");
+    if (P->n_tiles <= 0) return pfail(NLB_ERR_ARG, name);   // the tiles cover every amplitude
     F *M = static_cast<F*>(S->M), *W = static_cast<F*>(S->W), *Y = static_cast<F*>(S->Y);
     F *Xpp = static_cast<F*>(S->Xpp), *Xhh = static_cast<F*>(S->Xhh), *R = static_cast<F*>(S->R);
     F *U = static_cast<F*>(S->U), *G = static_cast<F*>(S->G), *H = static_cast<F*>(S->H);
     const int64_t nph = (int64_t)(4 * P->n_pmom) * (4 * P->n_hmom);
-    k_pw_xrow<F><<<pgrid(32 * P->n_rows), 256, 0, st>>>(*P, t2, Y);
+    k_pw_xrow<F><<<pgrid(16 * P->n_rows), 256, 0, st>>>(*P, t2, Y);
     k_pw_X<F><<<pgrid(32 * 16 * (int64_t)(P->n_pmom + P->n_hmom)), 256, 0, st>>>(*P, Y, M, Xpp, Xhh);
     k_pw_W<F><<<pgrid(P->n_w), 256, 0, st>>>(*P, M, W);
-    k_pw_R<F><<<pgrid(nph), 256, 0, st>>>(*P, t2, R, U, G);
+    k_pw_R<F><<<pgrid(16 * nph), 256, 0, st>>>(*P, t2, R, U, G);
     int rc = pcheck(name);
     if (rc != NLB_OK) return rc;
-    if (P->n_tiles > 0)
-        k_pw_residual<F><<<P->n_tiles < 65535 ? P->n_tiles : 65535, 256, 0, st>>>(*P, t2, M, W, Xpp, Xhh, R, U, G, H);
-    int64_t gx = 2 * ((P->n_t2 / P->n_blocks + 255) / 256);
-    gx = gx < 1 ? 1 : (gx > 64 ? 64 : gx);
-    k_pw_jacobi<F><<<dim3((unsigned)gx, (unsigned)P->n_blocks), 256, 0, st>>>(*P, t2, H, Xpp, Xhh, mixing, t2_out,
-                                                                            err);
+    const unsigned tiles = P->n_tiles < 65535 ? P->n_tiles : 65535;
+    k_pw_residual<F><<<tiles, 256, 0, st>>>(*P, t2, M, W, Xpp, Xhh, R, U, G, H);
+    k_pw_jacobi<F><<<tiles, 256, 0, st>>>(*P, t2, H, Xpp, Xhh, mixing, t2_out, err);
     return pcheck(name);
 }
 
