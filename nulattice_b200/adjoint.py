@@ -89,12 +89,20 @@ class LambdaSolver:
     multipliers, U, T and control block are written out in the layout of the
     full buffers."""
 
+    # fewest particles of a label for a run on one label: below, a step is
+    # launches only and the check of the amplitudes and the copies in and out
+    # cost more than they save (eight steps on one B200, one label against all:
+    # 20 particles, 7 sites 546 and 506 us; 26, 1 site 567 and 588 us; 57, 7
+    # sites 688 and 862 us; 124, 1 site 891 and 1564 us)
+    label_from = 24
+
     def __init__(self, eng):
         L = _lib.lib()
         self.eng = eng
         self.lattice = bool(L.nlb_lambda_lattice(eng.prob))
         self.n_gb = int(L.nlb_lambda_gb_len(eng.prob))
         self._label = None
+        self._ut = None
         self._bufs = {}
         self._coef = {}
 
@@ -214,7 +222,7 @@ class LambdaSolver:
         """(one-label solver, its start) when the amplitudes of ``b`` (and the
         multipliers, if kept) have the alike-label form, else None."""
         red = self.eng.reduced()
-        if red is None:
+        if red is None or red.plan.p < self.label_from:
             return None
         t1 = red.compress(b["t1"], b["t2"])
         lam1 = red.compress(b["lam1"][0], b["lam2"][0]) if keep and t1 is not None else None
@@ -239,10 +247,12 @@ class LambdaSolver:
         red._expand(r["lam1"][cur], b["lam1"][cur], r["lam2"][cur], b["lam2"][cur], False)
         # U and T of every label behind the Z1 accumulator, as in the full layout
         P, H = red.sizes
-        ut = torch.zeros((2, H, H), dtype=torch.float64, device=red.dev)
-        idx = red.orders[1].long().reshape(red.labels, h)
-        ut[:, idx[:, :, None], idx[:, None, :]] = r["acc"][p * h:p * h + 2 * h * h].reshape(2, 1, h, h)
-        b["acc"][P * H:P * H + 2 * H * H].copy_(ut.reshape(-1))
+        if self._ut is None:   # where the label's U and T entries go, label by label
+            idx = red.orders[1].long().reshape(red.labels, h)
+            ut = (idx[:, :, None] * H + idx[:, None, :]).reshape(1, red.labels, h * h)
+            self._ut = P * H + torch.cat([ut, ut + H * H]).reshape(-1)
+        b["acc"][P * H:P * H + 2 * H * H].zero_()
+        b["acc"][self._ut] = r["acc"][p * h:p * h + 2 * h * h].reshape(2, 1, h * h).expand(2, red.labels, h * h).reshape(-1)
         b["ctrl"].copy_(r["ctrl"])
         self.launches = solver.launches + 2
         return c
