@@ -1029,15 +1029,19 @@ __global__ void __launch_bounds__(kThreads) k_diis_reduce(nlb_ctrl* c, const dou
 // Leaves in gram[0] the weight of the current amplitudes and in gram[1+s]
 // the weight of error vector s (t_new = w0 t_m + sum_s w_s e_s).
 __global__ void k_diis_solve(nlb_ctrl* c) {
-    // one warp: lane t owns column t of the bordered matrix in shared memory;
-    // every entry sees the same operations in the same order as a serial
-    // elimination (partial pivoting, first maximum on ties)
+    // One warp.  Lane t owns column t of the bordered matrix in shared memory,
+    // and finds the pivot and the factors as row t: one division and
+    // three barriers per column (a division and two barriers per row: 13.0 us
+    // at eight vectors, all latency; 10.8 us this way, most of it the serial
+    // back substitution, whose order stays).  Every entry sees the same
+    // operations in the same order as a serial elimination (partial pivoting,
+    // first maximum on ties).
     if (blockIdx.x != 0 || !c->diis_pulse) return;
     const int lane = threadIdx.x;
     const int m = c->max_diis, n = m + 1;
     __shared__ double A[kMaxDiis + 1][kMaxDiis + 2];   // column n holds the right-hand side
     __shared__ double xs[kMaxDiis + 1];
-    __shared__ int s_ok;
+    __shared__ double fs[kMaxDiis + 1];                // factors of one column
     double mx = 0.0;
     for (int k = lane; k < m * m; k += 32) {
         const int s = k / m, t = k - s * m;
@@ -1055,36 +1059,48 @@ __global__ void k_diis_solve(nlb_ctrl* c) {
         else v = -1.0;
         A[s][t] = v;
     }
-    if (lane == 0) s_ok = 1;
     __syncwarp();
+    bool ok = true;
     for (int col = 0; col < n; ++col) {
-        if (lane == 0) {
-            int piv = col;
-            for (int r = col + 1; r < n; ++r)
-                if (fabs(A[r][col]) > fabs(A[piv][col])) piv = r;
-            if (A[piv][col] == 0.0 || !isfinite(A[piv][col])) s_ok = 0;
-            xs[0] = (double)piv;
+        // the serial scan keeps row col unless a later one is larger: a NaN
+        // there stays (and fails the test below), elsewhere it is passed over
+        const bool mine = lane >= col && lane < n;
+        const double own = mine ? A[lane][col] : 0.0;
+        double key = !mine ? -2.0 : own == own ? fabs(own) : lane == col ? INFINITY : -1.0;
+        int piv = lane;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double k2 = __shfl_xor_sync(0xffffffffu, key, o);
+            const int p2 = __shfl_xor_sync(0xffffffffu, piv, o);
+            if (k2 > key || (k2 == key && p2 < piv)) {
+                key = k2;
+                piv = p2;
+            }
+        }
+        const double pv = A[piv][col];
+        if (pv == 0.0 || !isfinite(pv)) {   // the same for every lane
+            ok = false;
+            break;
         }
         __syncwarp();
-        if (!s_ok) break;
-        const int piv = (int)xs[0];
         if (piv != col && lane <= n) {
             const double tmp = A[col][lane]; A[col][lane] = A[piv][lane]; A[piv][lane] = tmp;
         }
         __syncwarp();
-        for (int r = col + 1; r < n; ++r) {
-            const double f = A[r][col] / A[col][col];
-            __syncwarp();
-            if (lane >= col && lane <= n) A[r][lane] -= f * A[col][lane];
-            __syncwarp();
+        if (lane > col && lane < n) fs[lane] = A[lane][col] / pv;
+        __syncwarp();
+        if (lane >= col && lane <= n) {
+            const double top = A[col][lane];
+#pragma unroll 4
+            for (int r = col + 1; r < n; ++r) A[r][lane] -= fs[r] * top;
         }
+        __syncwarp();
     }
-    __syncwarp();
-    bool ok = s_ok != 0;
     if (lane == 0) {
         if (ok) {
             for (int r = n - 1; r >= 0; --r) {
                 double sum = A[r][n];
+#pragma unroll 4
                 for (int t = r + 1; t < n; ++t) sum -= A[r][t] * xs[t];
                 xs[r] = sum / A[r][r];
                 if (!isfinite(xs[r])) ok = false;
@@ -1110,7 +1126,7 @@ template <> struct Vec2<float> { using type = float2; };
 template <> struct Vec2<double> { using type = double2; };
 
 template <typename T, int M>
-__global__ void __launch_bounds__(kThreads) k_diis_extrap(nlb_struct_problem P, nlb_struct_state S) {
+__global__ void __launch_bounds__(kThreads) k_diis_extrap(nlb_struct_problem P, nlb_struct_state S, int both) {
     const nlb_ctrl* c = S.ctrl;
     if (!c->diis_pulse || !c->diis_applied) return;
     const int par = c->parity;
@@ -1134,6 +1150,25 @@ __global__ void __launch_bounds__(kThreads) k_diis_extrap(nlb_struct_problem P, 
     // T2: two amplitudes per thread with 8- (FP32) or 16-byte (FP64) loads
     // when every stored vector starts on such a boundary (n_t2 even, aligned
     // buffers); the arithmetic per amplitude is the same as one at a time
+    if (both) {
+        // t2 and the error vectors are symmetric bit for bit (k_sym_update wrote
+        // each pair a <= b in both places): read the pairs a <= b, write both
+        // (A=28 L=6 FP64, eight vectors: 31 -> 21 us, the same bits)
+        const unsigned nh = P.h, nhp = nh * nh, np = P.p;
+        for (int64_t q = tid; q < n2; q += stride) {
+            const unsigned ab = (unsigned)q / nhp, a = ab / np, b = ab - a * np;   // n2 < 2^31
+            if (b < a) continue;
+            double v = w0 * (double)t2[q];
+#pragma unroll
+            for (int s = 0; s < M; ++s) v += w[s] * (double)E2[(int64_t)s * P.n_t2 + q];
+            t2[q] = (T)v;
+            if (a != b) {
+                const unsigned hp = (unsigned)q - ab * nhp, i = hp / nh, j = hp - i * nh;
+                t2[((int64_t)b * np + a) * nhp + j * nh + i] = (T)v;
+            }
+        }
+        return;
+    }
     using V = typename Vec2<T>::type;
     const bool aligned = ((reinterpret_cast<uintptr_t>(t2) | reinterpret_cast<uintptr_t>(E2)) % sizeof(V)) == 0;
     const int64_t npair = (P.n_t2 % 2 == 0 && aligned) ? n2 / 2 : 0;
@@ -1530,7 +1565,8 @@ void diis_m(const nlb_struct_problem* P, const nlb_struct_state* S, cudaStream_t
     k_diis_gram<T, M><<<nb, kThreads, 0, st>>>(*P, *S);
     k_diis_reduce<M><<<M * (M + 1) / 2, kThreads, 0, st>>>(S->ctrl, prep_view(S->prep, *P).gram_slots(), nb);
     k_diis_solve<<<1, 32, 0, st>>>(S->ctrl);
-    k_diis_extrap<T, M><<<grid_for(k_diis_extrap<T, M>, (n + 1) / 2), kThreads, 0, st>>>(*P, *S);
+    k_diis_extrap<T, M><<<grid_for(k_diis_extrap<T, M>, (n + 1) / 2), kThreads, 0, st>>>(
+        *P, *S, use_sym<T>(P) && P->n_t2 < (int64_t(1) << 31));
     k_diis_done<<<1, 32, 0, st>>>(S->ctrl);
 }
 
