@@ -543,7 +543,10 @@ def main():
     # of the problem that runs: one channel when the labels are alike
     n_t2 = plan.n_t2
     work = eng.reduced() or eng
-    alg_bytes = (3 * work.plan.n_t2 + work.n_g) * 4
+    # two-launch steps: T2 read, written, error written (no Ga table); the
+    # events then span the row and the pair kernel
+    two = _lib.lib().nlb_struct_step_launches(work.prob, _lib.NLB_F32) == 2
+    alg_bytes = (3 * work.plan.n_t2 + (0 if two else work.n_g)) * 4
     k_ms = statistics.mean(m_k)
     achieved = alg_bytes / (k_ms * 1e-3) / 1e9
     peaks = {}
@@ -552,11 +555,13 @@ def main():
         peak, peak_src = float(peaks["hbm_gbs"]), "measured"
     except (OSError, KeyError, ValueError):
         peak, peak_src = 6650.0, "fallback"
+    kernel = "k_sym_row + k_sym_update" if two else T.t2_kernel_fp32(int(eng.prob.tune))
     traffic = None
     tfile = os.path.join(ROOT, "profiles", "t2_update_traffic.json")
     if os.path.exists(tfile):
-        traffic = json.load(open(tfile)).get("bytes_per_launch")
-    roofline = {"kernel": T.t2_kernel_fp32(int(eng.prob.tune)), "bound": "hbm", "achieved": achieved, "peak": peak,
+        rec = json.load(open(tfile))
+        traffic = rec.get("bytes_per_launch") if rec.get("kernel") == kernel else None
+    roofline = {"kernel": kernel, "bound": "hbm", "achieved": achieved, "peak": peak,
                 "peak_source": peak_src, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
                 "alg_bytes_per_launch": alg_bytes, "avg_launch_us": k_ms * 1e3, "launches": len(m_k)}
 

@@ -170,7 +170,11 @@ int nlb_struct_ctrl_init(nlb_ctrl *ctrl, double eps, double mixing, int32_t max_
 int nlb_struct_step(const nlb_struct_problem *prob, const nlb_struct_state *st,
                     nlb_stream_t stream);
 
-/* The five launches of nlb_struct_step one at a time (NLB_STAGE_*), so a
+/* Kernel launches of one nlb_struct_step: 2 for a label-symmetric problem that
+ * takes the row and pair kernels, else 4. */
+int nlb_struct_step_launches(const nlb_struct_problem *prob, int32_t dtype);
+
+/* The launches of nlb_struct_step one at a time (NLB_STAGE_*), so a
  * caller can bracket a single kernel with events.  Running the stages
  * PREP..FINISH in order is exactly one nlb_struct_step. */
 int nlb_struct_stage(const nlb_struct_problem *prob, const nlb_struct_state *st, int32_t stage,

@@ -141,6 +141,8 @@ def lib():
     L.nlb_struct_ctrl_init.argtypes = [c_void_p, c_double, c_double, c_int32, c_int32, c_int32, c_int32,
                                        c_double, c_void_p]
     L.nlb_struct_step.argtypes = [ctypes.POINTER(StructProblem), ctypes.POINTER(StructState), c_void_p]
+    L.nlb_struct_step_launches.argtypes = [ctypes.POINTER(StructProblem), c_int32]
+    L.nlb_struct_step_launches.restype = c_int32
     L.nlb_struct_diis.argtypes = [ctypes.POINTER(StructProblem), ctypes.POINTER(StructState), c_int32,
                                   c_void_p]
     L.nlb_struct_stage.argtypes = [ctypes.POINTER(StructProblem), ctypes.POINTER(StructState), c_int32,

@@ -442,14 +442,17 @@ class StructuredEngine:
             while chunk < 8:
                 chunk += max_diis
         use_graph = graph and not verbose and t2_events is None
+        per_step = L.nlb_struct_step_launches(self.prob, b["state"].dtype)
 
         def issue(n_steps, done0):
             for k in range(n_steps):
                 if t2_events is None:
                     _lib.check(L.nlb_struct_step(self.prob, st, sp), "step")
                 else:
+                    # on one label the row sums of T2 are the first stage
+                    first = _lib.NLB_STAGE_PREP if per_step == 2 else _lib.NLB_STAGE_T2
                     for stage in range(_lib.NLB_STAGE_PREP, _lib.NLB_STAGE_FINISH + 1):
-                        if stage == _lib.NLB_STAGE_T2:
+                        if stage == first:
                             ev0 = torch.cuda.Event(enable_timing=True)
                             ev1 = torch.cuda.Event(enable_timing=True)
                             ev0.record(stream)
@@ -457,7 +460,7 @@ class StructuredEngine:
                         if stage == _lib.NLB_STAGE_T2:
                             ev1.record(stream)
                             t2_events.append((ev0, ev1))
-                self.launches += 4   # prep+Ga, T2, T1, finish
+                self.launches += per_step   # row sums, pairs; or prep+Ga, T2, T1, finish
                 if use_diis and (done0 + k + 1) % max_diis == 0:
                     _lib.check(L.nlb_struct_diis(self.prob, st, max_diis, sp), "diis")
                     self.launches += 4
@@ -469,7 +472,7 @@ class StructuredEngine:
             if use_graph and n == chunk and b.get("warm"):
                 g = self._graph_for(b, chunk, max_diis if use_diis else 0, issue)
                 g.replay()
-                self.launches += (4 * chunk + (4 * (chunk // max_diis) if use_diis else 0))
+                self.launches += (per_step * chunk + (4 * (chunk // max_diis) if use_diis else 0))
             else:
                 issue(n, done)
                 b["warm"] = True
@@ -676,7 +679,8 @@ def solve_structured(eng, t1initial=None, eps=1e-8, maxSteps=1000, max_diis=10, 
             info["t_loop_build"] = eng.cache["t_loop_build"]
         iters = int(out[4])
         # kernels run: four per step, four per DIIS pulse, the prologue and report
-        eng.launches += 4 * iters + (4 * (iters // diis) if diis else 0) + 3
+        per_step = min(L.nlb_struct_step_launches(eng.prob, code) for code in (_lib.NLB_F32, _lib.NLB_F64))
+        eng.launches += per_step * iters + (4 * (iters // diis) if diis else 0) + 3
         if precision == "mixed":
             info["mixed_iters"] = int(out[7])
             info["mixed_energy"] = float(out[2])

@@ -1640,6 +1640,11 @@ int64_t nlb_struct_noalloc_scratch_bytes(const nlb_struct_problem* prob, int32_t
     return align256(nlb_struct_prep_len(prob) * 8) + align256(prob->n_g * el) + align256(prob->n_f2 * el);
 }
 
+int nlb_struct_step_launches(const nlb_struct_problem* prob, int32_t dtype) {
+    if (!prob) return 0;
+    return (dtype == NLB_F64 ? use_sym<double>(prob) : use_sym<float>(prob)) ? 2 : 4;
+}
+
 int nlb_struct_step_noalloc(const nlb_struct_problem* prob, const nlb_struct_state* st, nlb_stream_t stream) {
     if (!prob || !st || !st->ctrl) return fail(NLB_ERR_ARG, "nlb_struct_step_noalloc: null problem/state");
     if (st->dtype != NLB_F64 && st->dtype != NLB_F32) return fail(NLB_ERR_ARG, "nlb_struct_step_noalloc: bad dtype");
