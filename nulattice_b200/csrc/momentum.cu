@@ -307,12 +307,14 @@ __global__ void k_pw_W(nlb_pw_problem P, const F* __restrict__ M, F* __restrict_
 // Sixteen lanes per (a, i), one per result: sixteen holes k_k at a time, a lane
 // finds the amplitudes of one of them and every lane then adds its (s_c, s_k) of
 // each; G and U take R from the other lanes.  One thread per (a, i) left the SMs
-// with 0.6 blocks each: 24.5 us for A=28 L=6 FP64, 22.5 us this way (A=4 L=5 FP32: 11.5 and 4.9).
+// with 0.6 blocks each: 24.5 us for A=28 L=6 FP64, 15.2 us this way (A=4 L=5 FP32: 11.5 and 4.9 us).
 template <typename F>
 __global__ void __launch_bounds__(256) k_pw_R(nlb_pw_problem P, const F* __restrict__ t2, F* __restrict__ R,
                                               F* __restrict__ U, F* __restrict__ G) {
-    __shared__ F Vs[256];
-    for (int q = threadIdx.x; q < 256; q += blockDim.x) Vs[q] = P.V[q];
+    // V[x0][x1][x2][x3] at strides 84, 20, 4, 1: lanes that differ in x0 or x1 and
+    // x3 read different banks (at 64, 16, 4, 1 four of them share one)
+    __shared__ F Vs[4 * 84];
+    for (int q = threadIdx.x; q < 256; q += blockDim.x) Vs[(q >> 6) * 84 + ((q >> 4) & 3) * 20 + (q & 15)] = P.V[q];
     __syncthreads();
     const int L = P.L, L3 = L * L * L;
     const int nps = 4 * P.n_pmom, nhs = 4 * P.n_hmom;
@@ -350,8 +352,8 @@ __global__ void __launch_bounds__(256) k_pw_R(nlb_pw_problem P, const F* __restr
 #pragma unroll
             for (int sk = 0; sk < 4; ++sk) {
                 const F x = __shfl_sync(0xffffffffu, r, sc * 4 + sk, 16);
-                g += Vs[((hi * 4 + sk) * 4 + sc) * 4 + lo] * x;
-                u += Vs[((sc * 4 + hi) * 4 + sk) * 4 + lo] * x;
+                g += Vs[hi * 84 + sk * 20 + sc * 4 + lo] * x;
+                u += Vs[sc * 84 + hi * 20 + sk * 4 + lo] * x;
             }
         R[e * 16 + l] = r;
         G[e * 16 + l] = -g;
@@ -388,7 +390,7 @@ __device__ __forceinline__ float dot16(const float* __restrict__ x, const float*
 // each of their vectors once, as fragments straight from global memory (a
 // thread's four k are neighbours: the order of a sum over k is free).  One dot
 // product per amplitude read 512 bytes for each and kept the load unit busy 90%
-// of 181 us (A=28 L=6, 2.5 M amplitudes); 88.7 us this way.
+// of 181 us (A=28 L=6, 2.5 M amplitudes); 70.2 us this way, three blocks per SM (two: 88.7 us).
 constexpr int kTR = 64, kTC = 16;
 
 __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
@@ -409,7 +411,7 @@ __device__ __forceinline__ void frag16(const double* __restrict__ X, int64_t ld,
 }
 
 template <typename F>
-__global__ void __launch_bounds__(256) k_pw_residual(nlb_pw_problem P, const F* __restrict__ t2,
+__global__ void __launch_bounds__(256, 3) k_pw_residual(nlb_pw_problem P, const F* __restrict__ t2,
                                                      const F* __restrict__ M, const F* __restrict__ W,
                                                      const F* __restrict__ Xpp, const F* __restrict__ Xhh,
                                                      const F* __restrict__ R, const F* __restrict__ U,
