@@ -545,8 +545,8 @@ def main():
     work = eng.reduced() or eng
     # two-launch steps: T2 read, written, error written (no Ga table); the
     # events then span the row and the pair kernel
-    two = _lib.lib().nlb_struct_step_launches(work.prob, _lib.NLB_F32) == 2
-    alg_bytes = (3 * work.plan.n_t2 + (0 if two else work.n_g)) * 4
+    paired = _lib.lib().nlb_struct_step_launches(work.prob, _lib.NLB_F32) == 2
+    alg_bytes = (3 * work.plan.n_t2 + (0 if paired else work.n_g)) * 4
     k_ms = statistics.mean(m_k)
     achieved = alg_bytes / (k_ms * 1e-3) / 1e9
     peaks = {}
@@ -555,7 +555,7 @@ def main():
         peak, peak_src = float(peaks["hbm_gbs"]), "measured"
     except (OSError, KeyError, ValueError):
         peak, peak_src = 6650.0, "fallback"
-    kernel = "k_sym_row + k_sym_update" if two else T.t2_kernel_fp32(int(eng.prob.tune))
+    kernel = "k_sym_row + k_sym_update" if paired else T.t2_kernel_fp32(int(eng.prob.tune))
     traffic = None
     tfile = os.path.join(ROOT, "profiles", "t2_update_traffic.json")
     if os.path.exists(tfile):

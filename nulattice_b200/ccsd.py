@@ -75,6 +75,24 @@ def _resolve_device(device):
     return dev
 
 
+def _upload(arrays, device):
+    """Host arrays -> device tensors of their types and shapes in one buffer and
+    one copy (an allocation and a copy for each of some thirty small tables was
+    most of the time it takes to build an engine)."""
+    kinds = {np.dtype(np.int32): torch.int32, np.dtype(np.int64): torch.int64, np.dtype(np.float64): torch.float64,
+             np.dtype(np.uint8): torch.uint8}
+    at, end = {}, 0
+    for name, a in arrays.items():
+        at[name] = end
+        end += (a.nbytes + 255) // 256 * 256
+    host = np.zeros(max(end, 1), np.uint8)
+    for name, a in arrays.items():
+        host[at[name]:at[name] + a.nbytes] = a.reshape(-1).view(np.uint8)
+    buf = torch.as_tensor(host, device=device)
+    return {name: buf[at[name]:at[name] + a.nbytes].view(kinds[a.dtype]).reshape(a.shape)
+            for name, a in arrays.items()}
+
+
 class StructuredEngine:
     """Device tables and buffers of one structured problem.
 
@@ -207,9 +225,9 @@ class StructuredEngine:
         device = self.dev
         G = pl.n_labels
         dev = device
-        i32 = lambda a: torch.as_tensor(np.ascontiguousarray(a, dtype=np.int32), device=dev)  # noqa: E731
-        i64 = lambda a: torch.as_tensor(np.ascontiguousarray(a, dtype=np.int64), device=dev)  # noqa: E731
-        f64 = lambda a: torch.as_tensor(np.ascontiguousarray(a, dtype=np.float64), device=dev)  # noqa: E731
+        i32 = lambda a: np.ascontiguousarray(a, dtype=np.int32)  # noqa: E731
+        i64 = lambda a: np.ascontiguousarray(a, dtype=np.int64)  # noqa: E731
+        f64 = lambda a: np.ascontiguousarray(a, dtype=np.float64)  # noqa: E731
         p_ord = np.concatenate([pl.p_of[g] for g in range(G)]).astype(np.int32)
         h_ord = np.concatenate([pl.h_of[g] for g in range(G)]).astype(np.int32)
         chans = np.zeros(max(len(pl.channels), 1), dtype=_lib.CHANNEL_DTYPE)
@@ -242,7 +260,7 @@ class StructuredEngine:
         self.n_t1c, self.n_xc = int(t1c_base[-1]), int(xc_base[-1])
         cat = lambda xs, dt: np.concatenate(xs).astype(dt) if xs else np.zeros(1, dt)  # noqa: E731
         T = {}
-        T["chan"] = torch.as_tensor(chans.view(np.uint8), device=dev)
+        T["chan"] = chans.view(np.uint8)
         T["t2_end"] = i64(t2_end or [0]); T["g_end"] = i64(g_end or [0]); T["row_end"] = i64(row_end or [0])
         T["t1c_base"] = i32(t1c_base); T["xc_base"] = i32(xc_base)
         T["p_ord"] = i32(p_ord); T["h_ord"] = i32(h_ord)
@@ -275,7 +293,7 @@ class StructuredEngine:
             xc_ki.append((H_[:, None] * pl.h + H_[None, :]).ravel())
         T["t1c_idx"] = i32(cat(t1c_idx, np.int64))
         T["xc_ki"] = i32(cat(xc_ki, np.int64))
-        self._tables = T
+        T = self._tables = _upload(T, dev)
         prob = _lib.StructProblem()
         prob.p, prob.h, prob.n_labels, prob.n_channels = pl.p, pl.h, G, len(pl.channels)
         prob.n_t2, prob.n_g, prob.n_f2, prob.n_rows = pl.n_t2, self.n_g, self.n_f2, self.n_rows
