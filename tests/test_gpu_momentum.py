@@ -121,3 +121,28 @@ def test_fp32_step_tracks_the_fp64_step():
     assert E32 == pytest.approx(E64, rel=1e-6)
     scale = float(y64.abs().max())
     assert float((y32.double() - y64).abs().max()) <= 1e-5 * scale
+
+
+@pytest.mark.parametrize("precision,eps", [("fp64", 2.0 ** -53), ("mixed", 2.0 ** -24)])
+def test_steps_with_more_holes_than_a_group_of_lanes(precision, eps):
+    """Nineteen hole momenta (all with components of at most one, two of them
+    not zero) at L=3: the ring sums take two rounds of sixteen holes, the blocks
+    have row and column remainders.  Two steps against the same steps in NumPy;
+    a step's longest sums have 16 * 19 products of terms no larger than the
+    result's largest element, eight for what cancels."""
+    import itertools
+    import momentum_model as MM
+    L = 3
+    ks = [k for k in itertools.product((0, 1, -1), repeat=3) if sum(x * x for x in k) <= 2]
+    plan = MB.MomentumPlan(L, [[*(x % L for x in k), tz, sz] for k in ks for tz in range(2) for sz in range(2)])
+    V = MB.contact_tensor(L, plan.n_k, -0.6, -0.5, 0.1)
+    fpp, fhh, _ = MB.fock_blocks(L, plan.n_k, plan.hmom, plan.pmom, -0.6, -0.5, 0.1)
+    eng = MB.MomentumEngine(plan, V, fpp, fhh, DEV)
+    got = [MB.solve(plan, V, fpp, fhh, eps=0.0, mixed_eps=0.0, maxSteps=n, max_diis=0, criterion="numpy", engine=eng,
+                    precision=precision)[1] for n in (1, 3)]
+    got = [np.asarray(x.double().cpu() if torch.is_tensor(x) else x, dtype=np.float64).reshape(-1) for x in got]
+    want = got[0]
+    for _ in range(2):
+        want = MM.step(plan, V, fpp, fhh, want)
+    assert np.abs(want - got[0]).max() > 1e-3 * np.abs(want).max()
+    assert np.abs(got[1] - want).max() <= 2 * 8 * 304 * eps * np.abs(want).max()
