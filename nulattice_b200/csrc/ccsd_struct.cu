@@ -937,14 +937,16 @@ __global__ void __launch_bounds__(kFinishThreads) k_finish(nlb_ctrl* c, const do
 // the dense t2 (four images per stored amplitude).
 constexpr int kMaxDiis = 10;
 
-template <typename T, int M>
+// A: type of the products and of a thread's sums (block and grid sums are
+// FP64).  The vectors are nearly parallel, so the solved weights, and with them
+// the step at which the energy test ends an FP32 phase, hang on these roundings.
+// FP32 vectors of one label for all: FP64 (40 couplings each at A=4 and 28,
+// L=3-5, mixed solves to 1e-12: 25-30 iterations on average against 28-33 with
+// FP32).  FP32 vectors of every label: FP32, the sums that the mixed solves with
+// an FP64 finish are pinned to (see solve_structured).  FP64 vectors: FP64.  Two
+// elements per thread and step keep 2M loads in flight.
+template <typename T, int M, typename A>
 __global__ void __launch_bounds__(kThreads) k_diis_gram(nlb_struct_problem P, nlb_struct_state S) {
-    // Products and sums in FP64 for either vector type: the vectors are nearly
-    // parallel, and an FP32 sum's 1e-6 costs the extrapolation digits (40
-    // couplings each at A=4 and 28, L=3-5, mixed solves to 1e-12: 25-30
-    // iterations on average against 28-33 with FP32 sums).  Two elements per
-    // thread and step keep 2M loads in flight.
-    using A = double;
     nlb_ctrl* c = S.ctrl;
     if (!c->diis_pulse) return;
     constexpr int NP = M * (M + 1) / 2;
@@ -1560,9 +1562,10 @@ int step_t(const nlb_struct_problem* P, const nlb_struct_state* S, cudaStream_t 
 template <typename T, int M>
 void diis_m(const nlb_struct_problem* P, const nlb_struct_state* S, cudaStream_t st) {
     const int64_t n = (int64_t)P->p * P->h + P->n_t2;
-    int nb = grid_for(k_diis_gram<T, M>, n);
+    auto gram = sym_labels(*P) > 1 ? k_diis_gram<T, M, double> : k_diis_gram<T, M, T>;
+    int nb = grid_for(gram, n);
     if (nb > kGramSlots) nb = kGramSlots;
-    k_diis_gram<T, M><<<nb, kThreads, 0, st>>>(*P, *S);
+    gram<<<nb, kThreads, 0, st>>>(*P, *S);
     k_diis_reduce<M><<<M * (M + 1) / 2, kThreads, 0, st>>>(S->ctrl, prep_view(S->prep, *P).gram_slots(), nb);
     k_diis_solve<<<1, 32, 0, st>>>(S->ctrl);
     k_diis_extrap<T, M><<<grid_for(k_diis_extrap<T, M>, (n + 1) / 2), kThreads, 0, st>>>(

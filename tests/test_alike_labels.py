@@ -11,6 +11,7 @@ from nulattice_b200 import _lib
 from nulattice_b200 import adjoint as A
 from nulattice_b200 import hamiltonian as ham
 from nulattice_b200 import structure as S
+from nulattice_b200 import tune
 from nulattice_b200.ccsd import StructuredEngine, solve_structured
 
 SEVEN = [(0, 0, 0), (1, 0, 0), (-1, 0, 0), (0, 1, 0), (0, -1, 0), (0, 0, 1), (0, 0, -1)]
@@ -110,6 +111,38 @@ def test_step_kernels_over_hole_counts_and_row_lengths(L, sites, precision, eps)
         out[full] = e, t1.cpu().numpy(), t2.double().cpu().numpy()
     for got, want in zip(out[False], out[True]):
         assert np.abs(np.asarray(got) - want).max() <= 3 * 8 * (16 + 4 * sites) * eps * np.abs(want).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,sites,C2,C3,steps", [(3, 2, -3.1, 0.9, (18, 28)), (3, 7, -2.9, 0.6, (15, 29)),
+                                                 (4, 7, -3.1, 0.9, (12, 30)), (4, 7, -3.3, 0.7, (12, 27)),
+                                                 (4, 2, -3.0, 1.0, (15, 33)), (6, 7, -3.1, 0.9, (12, 30))])
+@pytest.mark.parametrize("loop", ["eager", "graph"])
+def test_mixed_solves_to_fp64_keep_every_label(L, sites, C2, C3, steps, loop):
+    """Where the energy test stops such a solve hangs on the roundings of its FP32
+    pulses: it runs on every label, bit for bit what the kernels for every label
+    give, and its (FP32, all) step counts on a B200 are those it had before labels
+    were reduced."""
+    _, fock, two = _inputs(L, sites, C2, C3)
+    plan, _ = S.detect(fock, two)
+    out = []
+    for full in (False, True):
+        eng = StructuredEngine(plan, fock, torch.device("cuda:0"))
+        eng.prob.tune = tune.known_word(eng)
+        if full:
+            eng.cache["reduced"] = None
+        info = {}
+        out.append(solve_structured(eng, eps=1e-11, mixed_eps=1e-6, maxSteps=100, max_diis=8, precision="mixed",
+                                    t2_format="compact", loop=loop, info=info))
+        assert info["n_t2_stored"] == eng.plan.n_t2
+        assert (info["mixed_iters"], info["iterations"]) == steps
+    assert out[0][0] == out[1][0] and torch.equal(out[0][1], out[1][1]) and torch.equal(out[0][2], out[1][2])
+    # an answer of the FP32 phase alone, and a phase too short for a pulse, run on one label
+    for kw in (dict(eps=1e-6), dict(eps=1e-11, refine=False), dict(eps=1e-11, maxSteps=7)):
+        eng = StructuredEngine(plan, fock, torch.device("cuda:0"))
+        solve_structured(eng, mixed_eps=1e-6, max_diis=8, precision="mixed", t2_format="compact", loop="eager",
+                         info=info, **kw)
+        assert info["n_t2_stored"] == plan.n_t2 // 6
 
 
 @pytest.mark.gpu
