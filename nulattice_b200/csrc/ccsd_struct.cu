@@ -1559,8 +1559,9 @@ int step_t(const nlb_struct_problem* P, const nlb_struct_state* S, cudaStream_t 
     return check_launch("nlb_struct_step");
 }
 
+// both: t2 and the error vectors are symmetric bit for bit (k_diis_extrap).
 template <typename T, int M>
-void diis_m(const nlb_struct_problem* P, const nlb_struct_state* S, cudaStream_t st) {
+void diis_m(const nlb_struct_problem* P, const nlb_struct_state* S, int both, cudaStream_t st) {
     const int64_t n = (int64_t)P->p * P->h + P->n_t2;
     auto gram = sym_labels(*P) > 1 ? k_diis_gram<T, M, double> : k_diis_gram<T, M, T>;
     int nb = grid_for(gram, n);
@@ -1568,24 +1569,27 @@ void diis_m(const nlb_struct_problem* P, const nlb_struct_state* S, cudaStream_t
     gram<<<nb, kThreads, 0, st>>>(*P, *S);
     k_diis_reduce<M><<<M * (M + 1) / 2, kThreads, 0, st>>>(S->ctrl, prep_view(S->prep, *P).gram_slots(), nb);
     k_diis_solve<<<1, 32, 0, st>>>(S->ctrl);
-    k_diis_extrap<T, M><<<grid_for(k_diis_extrap<T, M>, (n + 1) / 2), kThreads, 0, st>>>(
-        *P, *S, use_sym<T>(P) && P->n_t2 < (int64_t(1) << 31));
+    k_diis_extrap<T, M><<<grid_for(k_diis_extrap<T, M>, (n + 1) / 2), kThreads, 0, st>>>(*P, *S, both);
     k_diis_done<<<1, 32, 0, st>>>(S->ctrl);
 }
 
+// forward: the vectors are those of forward steps.  k_sym_update writes a pair
+// in both places; the Lambda kernels form the two halves of a block one by one,
+// equal to rounding only.
 template <typename T>
-int diis_t(const nlb_struct_problem* P, const nlb_struct_state* S, int m, cudaStream_t st) {
+int diis_t(const nlb_struct_problem* P, const nlb_struct_state* S, int m, bool forward, cudaStream_t st) {
+    const int both = forward && use_sym<T>(P) && P->n_t2 < (int64_t(1) << 31);
     switch (m) {
-        case 1: diis_m<T, 1>(P, S, st); break;
-        case 2: diis_m<T, 2>(P, S, st); break;
-        case 3: diis_m<T, 3>(P, S, st); break;
-        case 4: diis_m<T, 4>(P, S, st); break;
-        case 5: diis_m<T, 5>(P, S, st); break;
-        case 6: diis_m<T, 6>(P, S, st); break;
-        case 7: diis_m<T, 7>(P, S, st); break;
-        case 8: diis_m<T, 8>(P, S, st); break;
-        case 9: diis_m<T, 9>(P, S, st); break;
-        case 10: diis_m<T, 10>(P, S, st); break;
+        case 1: diis_m<T, 1>(P, S, both, st); break;
+        case 2: diis_m<T, 2>(P, S, both, st); break;
+        case 3: diis_m<T, 3>(P, S, both, st); break;
+        case 4: diis_m<T, 4>(P, S, both, st); break;
+        case 5: diis_m<T, 5>(P, S, both, st); break;
+        case 6: diis_m<T, 6>(P, S, both, st); break;
+        case 7: diis_m<T, 7>(P, S, both, st); break;
+        case 8: diis_m<T, 8>(P, S, both, st); break;
+        case 9: diis_m<T, 9>(P, S, both, st); break;
+        case 10: diis_m<T, 10>(P, S, both, st); break;
         default: return fail(NLB_ERR_ARG, "max_diis must be in [1, 10]");
     }
     return check_launch("nlb_struct_diis");
@@ -1631,7 +1635,29 @@ int noalloc_scratch(void** out) {
 }
 
 int64_t align256(int64_t b) { return (b + 255) & ~int64_t(255); }
+
+int struct_diis(const nlb_struct_problem* prob, const nlb_struct_state* st, int32_t max_diis, bool forward,
+                nlb_stream_t stream) {
+    // reads the amplitudes, the rings and the partial-sum area of st->prep
+    // (not st->g / st->f2)
+    if (!prob || !st || !st->ctrl) return fail(NLB_ERR_ARG, "nlb_struct_diis: null problem/state");
+    if (prob->p <= 0 || prob->h <= 0 || prob->n_t2 < 0) return fail(NLB_ERR_SIZE, "nlb_struct_diis: bad sizes");
+    if (st->dtype != NLB_F64 && st->dtype != NLB_F32) return fail(NLB_ERR_ARG, "nlb_struct_diis: bad dtype");
+    if (!st->t1[0] || !st->t1[1] || !st->prep) return fail(NLB_ERR_ARG, "nlb_struct_diis: null t1/prep buffer");
+    if (prob->n_t2 > 0 && (!st->t2[0] || !st->t2[1])) return fail(NLB_ERR_ARG, "nlb_struct_diis: null t2 buffer");
+    if (!st->diis_t1 || (prob->n_t2 > 0 && !st->diis_t2)) return fail(NLB_ERR_ARG, "null DIIS ring");
+    if (max_diis < 1 || max_diis > kMaxDiis) return fail(NLB_ERR_ARG, "max_diis must be in [1, 10]");
+    cudaStream_t s = (cudaStream_t)stream;
+    return st->dtype == NLB_F64 ? diis_t<double>(prob, st, max_diis, forward, s) : diis_t<float>(prob, st, max_diis, forward, s);
+}
+
 }  // namespace
+
+// The pulse of the Lambda iteration (lambda.cu): `st` is a view of the multipliers.
+int nlb_internal_lambda_diis(const nlb_struct_problem* prob, const nlb_struct_state* st, int32_t max_diis,
+                             nlb_stream_t stream) {
+    return struct_diis(prob, st, max_diis, false, stream);
+}
 
 extern "C" {
 
@@ -1723,17 +1749,7 @@ int nlb_struct_stage(const nlb_struct_problem* prob, const nlb_struct_state* st,
 
 int nlb_struct_diis(const nlb_struct_problem* prob, const nlb_struct_state* st, int32_t max_diis,
                     nlb_stream_t stream) {
-    // reads the amplitudes, the rings and the partial-sum area of st->prep
-    // (not st->g / st->f2)
-    if (!prob || !st || !st->ctrl) return fail(NLB_ERR_ARG, "nlb_struct_diis: null problem/state");
-    if (prob->p <= 0 || prob->h <= 0 || prob->n_t2 < 0) return fail(NLB_ERR_SIZE, "nlb_struct_diis: bad sizes");
-    if (st->dtype != NLB_F64 && st->dtype != NLB_F32) return fail(NLB_ERR_ARG, "nlb_struct_diis: bad dtype");
-    if (!st->t1[0] || !st->t1[1] || !st->prep) return fail(NLB_ERR_ARG, "nlb_struct_diis: null t1/prep buffer");
-    if (prob->n_t2 > 0 && (!st->t2[0] || !st->t2[1])) return fail(NLB_ERR_ARG, "nlb_struct_diis: null t2 buffer");
-    if (!st->diis_t1 || (prob->n_t2 > 0 && !st->diis_t2)) return fail(NLB_ERR_ARG, "null DIIS ring");
-    if (max_diis < 1 || max_diis > kMaxDiis) return fail(NLB_ERR_ARG, "max_diis must be in [1, 10]");
-    cudaStream_t s = (cudaStream_t)stream;
-    return st->dtype == NLB_F64 ? diis_t<double>(prob, st, max_diis, s) : diis_t<float>(prob, st, max_diis, s);
+    return struct_diis(prob, st, max_diis, true, stream);
 }
 
 int nlb_struct_energy(const nlb_struct_problem* prob, const nlb_struct_state* st, double* e_out,

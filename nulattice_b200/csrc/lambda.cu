@@ -30,6 +30,8 @@
 #include "nulattice_b200.h"
 
 void nlb_internal_set_error(const char* msg);
+int nlb_internal_lambda_diis(const nlb_struct_problem* prob, const nlb_struct_state* st, int32_t max_diis,
+                             nlb_stream_t stream);
 
 namespace {
 
@@ -1365,7 +1367,7 @@ int nlb_lambda_diis(const nlb_struct_problem* prob, const nlb_lambda_state* st, 
     v.diis_t1 = st->diis_t1;
     v.diis_t2 = st->diis_t2;
     v.dtype = st->dtype;
-    return nlb_struct_diis(prob, &v, max_diis, stream);
+    return nlb_internal_lambda_diis(prob, &v, max_diis, stream);
 }
 
 int nlb_lambda_coupling(const nlb_struct_problem* prob, const nlb_lambda_state* st, const double* dw,

@@ -201,3 +201,32 @@ def test_gradient_on_one_label(L, sites, precision):
         _, t1, t2 = solve_structured(eng, eps=1e-13, max_diis=8, maxSteps=2000, t2_format="compact")
         grads.append(A.lambda_gradient(eng, t1, t2, [prob.dv, prob.dw], tol=1e-10, precision=precision))
     np.testing.assert_allclose(grads[0], grads[1], rtol=1e-8)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,sites,code,eps", [(3, 2, _lib.NLB_F64, 2.0 ** -53), (3, 7, _lib.NLB_F64, 2.0 ** -53),
+                                              (4, 7, _lib.NLB_F32, 2.0 ** -24)])
+def test_lambda_pulse_extrapolates_every_entry(L, sites, code, eps):
+    """A pulse of the Lambda iteration on one label, from multipliers without
+    exchange symmetry: every entry is the same combination of its own last value
+    and its own stored errors.  The weights come from the pulse's t1 part, as those
+    that fit it best; FP32: the result is rounded once."""
+    _, eng = _engine(L, sites)
+    red = eng.reduced()
+    solver = A.LambdaSolver(red)
+    b = solver.buffers(code, 2)
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    for x in (b["t1"], b["t2"], b["lam1"][0], b["lam2"][0]):
+        x.copy_(torch.randn(x.shape, generator=gen, device="cuda", dtype=torch.float64) * 0.1)
+    lib, sp = _lib.lib(), torch.cuda.current_stream().cuda_stream
+    _lib.check(lib.nlb_lambda_init(red.prob, b["state"], 0.0, 0.5, 100, 2, _lib.NLB_LAMBDA_KEEP, sp), "init")
+    for _ in range(2):
+        _lib.check(lib.nlb_lambda_step(red.prob, b["state"], sp), "step")
+    before = b["lam1"][0].cpu().numpy(), b["lam2"][0].double().cpu().numpy()   # two steps: parity 0 again
+    e1, e2 = b["diis_t1"].view(2, -1).cpu().numpy(), b["diis_t2"].view(2, -1).double().cpu().numpy()
+    _lib.check(lib.nlb_lambda_diis(red.prob, b["state"], 2, sp), "diis")
+    after = b["lam1"][0].cpu().numpy(), b["lam2"][0].double().cpu().numpy()
+    w = np.linalg.lstsq(np.stack([before[0], *e1], 1), after[0], rcond=None)[0]
+    assert np.abs(w[1:]).max() > 1e-3      # the pulse did something
+    want = np.tensordot(w, np.stack([before[1], *e2]), 1)
+    assert np.abs(after[1] - want).max() <= (eps + 1e-11) * max(1.0, np.abs(want).max())
