@@ -516,7 +516,9 @@ __global__ void k_l_init(nlb_ctrl* c, double tol, double mixing, int max_steps, 
 }
 
 // <Lam, (dW + dV) tau> over the compact layout for a derivative Hamiltonian
-// whose ladders are diagonal: dw[hh_ptr_off + hp], dv[pp_ptr_off + ab].
+// whose ladders are diagonal: dw[hh_ptr_off + hp], dv[pp_ptr_off + ab].  Reads
+// the state's own t1, t2 and multipliers (of prep only the slots it writes), so
+// it holds whichever buffers the iteration ran on.
 __global__ void k_l_coupling(nlb_struct_problem P, nlb_lambda_state S, const double* dw, const double* dv,
                              double* out) {
     const double* Lm = static_cast<const double*>(S.lam2[S.ctrl->parity]);
@@ -550,8 +552,8 @@ __global__ void k_l_coupling(nlb_struct_problem P, nlb_lambda_state S, const dou
             }
             const int bp = e / nhp, hp = e - bp * nhp;
             const int ip = hp / ch->nh2, jp = hp - ip * ch->nh2;
-            const double tau = t2[u] + PV.t1c[P.t1c_base[ch->g1] + ap * ch->nh1 + ip] *
-                                           PV.t1c[P.t1c_base[ch->g2] + bp * ch->nh2 + jp];
+            const double tau = t2[u] + S.t1[(int64_t)P.p_ord[ch->pb1 + ap] * P.h + P.h_ord[ch->hb1 + ip]] *
+                                           S.t1[(int64_t)P.p_ord[ch->pb2 + bp] * P.h + P.h_ord[ch->hb2 + jp]];
             acc += Lm[u] * (dw[ch->hh_ptr_off + hp] + dv[ch->pp_ptr_off + ap * ch->np2 + bp]) * tau;
         }
     }

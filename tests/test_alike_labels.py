@@ -128,7 +128,7 @@ def test_mixed_solves_to_fp64_keep_every_label(L, sites, C2, C3, steps, loop):
     out = []
     for full in (False, True):
         eng = StructuredEngine(plan, fock, torch.device("cuda:0"))
-        eng.prob.tune = tune.known_word(eng)
+        eng.prob.tune = tune.word(fwd32=6, chunks=2)   # the roundings are those of one launch shape
         if full:
             eng.cache["reduced"] = None
         info = {}
@@ -230,3 +230,24 @@ def test_lambda_pulse_extrapolates_every_entry(L, sites, code, eps):
     assert np.abs(w[1:]).max() > 1e-3      # the pulse did something
     want = np.tensordot(w, np.stack([before[1], *e2]), 1)
     assert np.abs(after[1] - want).max() <= (eps + 1e-11) * max(1.0, np.abs(want).max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,sites", [(3, 3), (4, 7)])
+def test_derivative_that_treats_labels_differently(L, sites):
+    """Alike amplitudes and a derivative Hamiltonian with one pair of labels apart:
+    the multipliers may run on one label, the coupling sums take all of them."""
+    grads = []
+    for full in (False, True):
+        holes, eng = _engine(L, sites, full)
+        prob = A.lattice_problem(L, holes)
+        de, dfock, dtwo = prob.dv
+        idx, val = (np.asarray(x) for x in S._coo(dtwo[0]))
+        one = np.isin(eng.plan.p_label[idx[:, :2]], (0, 1)).all(1)    # v_pppp of labels 0 and 1 only, doubled
+        dtwo = [(idx, np.where(one, 2.0, 1.0) * val)] + list(dtwo[1:])
+        _, t1, t2 = solve_structured(eng, eps=1e-13, max_diis=8, maxSteps=2000, t2_format="compact")
+        if not full:
+            start = t1, t2
+            assert A._label_coefficients(eng.reduced(), dfock, dtwo) is None
+        grads.append(A.lambda_gradient(eng, *start, [(de, dfock, dtwo), prob.dw], tol=1e-11, precision="fp64"))
+    np.testing.assert_allclose(grads[0], grads[1], rtol=1e-9)
