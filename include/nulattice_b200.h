@@ -236,7 +236,7 @@ int nlb_struct_pack_t2(const nlb_struct_problem *prob, const double *t2_dense, v
  *
  * nlb_sym_check: do amplitudes of the full layout (t1 [mp * mh], compact t2 of
  * all pairs of labels) have the symmetric form?  out (device, 3 words):
- * [0] != 0 when labels differ; [1], [2] the bits of the largest
+ * [0] != 0 when labels differ or a value is NaN; [1], [2] the bits of the largest
  * |B[a,b,i,j] - B[b,a,j,i]| and |B[a,b,i,j]| of the first block.  t1_out
  * (optional, [p*h]) receives t1 of the first label.
  * nlb_sym_expand: the full layout from the stored parts: t1 (or NULL), and t2

@@ -205,19 +205,18 @@ class StructuredEngine:
 
     def compress(self, t1_full, t2_full):
         """t1 of one label when amplitudes of the full layout (device, t2
-        compact) have the alike-label form -- labels bit for bit, exchange
-        to rounding -- else None.  The first block of ``t2_full`` is then t2."""
+        compact) have the alike-label form -- labels and exchange bit for bit, as
+        the steps of one label leave them -- else None.  The first block of
+        ``t2_full`` is then t2."""
         t1 = torch.empty(self.plan.p * self.plan.h, dtype=torch.float64, device=self.dev)
         out = torch.empty(3, dtype=torch.int64, device=self.dev)
-        f32 = t2_full.dtype == torch.float32
+        code = _lib.NLB_F32 if t2_full.dtype == torch.float32 else _lib.NLB_F64
         _lib.check(_lib.lib().nlb_sym_check(self.prob, self.orders[0].data_ptr(), self.orders[1].data_ptr(),
-                                            t1_full.data_ptr(), t2_full.data_ptr(),
-                                            _lib.NLB_F32 if f32 else _lib.NLB_F64, t1.data_ptr(), out.data_ptr(),
-                                            _stream_ptr(self.dev)), "check")
+                                            t1_full.data_ptr(), t2_full.data_ptr(), code, t1.data_ptr(),
+                                            out.data_ptr(), _stream_ptr(self.dev)), "check")
         self.launches += 1
         o = out.cpu().numpy()
-        bad, (asym, big) = int(o[0]), o[1:].view(np.float64)
-        return t1 if bad == 0 and asym <= (1e-5 if f32 else 1e-8) * big else None
+        return t1 if o[0] == 0 and o[1] == 0 else None
 
     def _build(self):
         pl = self.plan

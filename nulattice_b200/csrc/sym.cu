@@ -45,7 +45,7 @@ struct Orders {
     const int32_t *p, *h;
 };
 
-// out[0] != 0: t1 or t2 differs between labels, or t1 joins two labels;
+// out[0] != 0: t1 or t2 differs between labels or is NaN, or t1 joins two labels;
 // out[1], out[2]: largest |B[a,b,i,j] - B[b,a,j,i]| and |B[a,b,i,j]| of the
 // block, as the bit patterns of non-negative doubles (which order like them);
 // t1_out (optional): t1 of the first label.
@@ -59,6 +59,7 @@ __global__ void __launch_bounds__(kT) k_sym_check(int m, int np, int nh, Orders 
     double asym = 0.0, big = 0.0;
     for (int64_t e = tid; e < n0; e += stride) {
         const T v = t2[e];
+        bad |= v != v;
         for (int c = 1; c < pairs; ++c) bad |= !(t2[c * n0 + e] == v);
         const int ab = (int)(e / (nh * nh)), ij = (int)(e - (int64_t)ab * nh * nh);
         const int a = ab / np, b = ab - a * np, i = ij / nh, j = ij - i * nh;
@@ -70,7 +71,7 @@ __global__ void __launch_bounds__(kT) k_sym_check(int m, int np, int nh, Orders 
         const int g = x / np, gh = y / nh;
         const double v = t1[(int64_t)o.p[x] * H + o.h[y]];
         if (g != gh) bad |= v != 0.0;
-        else bad |= !(v == t1[(int64_t)o.p[x - g * np] * H + o.h[y - g * nh]]);
+        else bad |= !(v == t1[(int64_t)o.p[x - g * np] * H + o.h[y - g * nh]]);   // label 0: NaN alone
     }
     if (t1_out)
         for (int64_t u = tid; u < nb; u += stride) t1_out[u] = t1[(int64_t)o.p[u / nh] * H + o.h[u % nh]];

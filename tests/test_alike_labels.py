@@ -251,3 +251,49 @@ def test_derivative_that_treats_labels_differently(L, sites):
             assert A._label_coefficients(eng.reduced(), dfock, dtwo) is None
         grads.append(A.lambda_gradient(eng, *start, [(de, dfock, dtwo), prob.dw], tol=1e-11, precision="fp64"))
     np.testing.assert_allclose(grads[0], grads[1], rtol=1e-9)
+
+
+def _labels(fock, two, keep):
+    """The inputs of some of the labels: Fock blocks and ladders of their states."""
+    plan, _ = S.detect(fock, two)
+    P, H = (np.flatnonzero(np.isin(x, keep)) for x in (plan.p_label, plan.h_label))
+    ladders = []
+    for block, states in ((two[0], P), (two[5], H)):
+        idx, val = S._coo(block)
+        m = np.isin(idx, states).all(1)
+        ladders.append((np.searchsorted(states, idx[m]), val[m]))
+    return [fock[0][np.ix_(P, P)], fock[1][np.ix_(P, H)], fock[2][np.ix_(H, H)]], \
+        [ladders[0]] + list(two[1:5]) + [ladders[1]]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,step", [(torch.float64, 1e-12), (torch.float32, 1e-6)])
+def test_amplitudes_count_as_alike_bit_for_bit(dtype, step):
+    """Labels that differ, an exchange that does not hold to the last bit, and a NaN
+    are each seen, also where two labels leave one block and no copy to compare."""
+    holes, fock, two = _inputs(3, 3)
+    for keep in ([0, 1, 2, 3], [0, 1]):
+        f, t = _labels(fock, two, keep)
+        plan, why = S.detect(f, t)
+        eng = StructuredEngine(plan, f, torch.device("cuda:0"))
+        red = eng.reduced()
+        assert red.labels == len(keep)
+        _, t1, t2 = solve_structured(eng, eps=1e-12, max_diis=8, t2_format="compact")
+        t2 = t2.to(dtype)
+        np.testing.assert_array_equal(red.compress(t1, t2).cpu().numpy(),
+                                      t1.cpu().numpy()[np.ix_(plan.p_of[0], plan.h_of[0])].ravel())
+        n = red.plan.n_t2
+        for value in (1.0 + step, float("nan")):
+            x = t2.clone()
+            k = red.plan.h ** 2                   # a = 0, b = 1, i = j = 0
+            assert x[k] != 0
+            x.view(-1, n)[:, k] *= value          # the same in every pair of labels
+            assert red.compress(t1, x) is None
+        x, y = t2.clone(), t1.clone()
+        x[-1] += 1.0
+        y[plan.p_of[1][0], plan.h_of[1][0]] += 1e-15
+        assert len(keep) == 2 or red.compress(t1, x) is None
+        assert red.compress(y, t2) is None
+        y = t1.clone()
+        y[plan.p_of[0][1], plan.h_of[0][0]] = float("nan")
+        assert red.compress(y, t2) is None
