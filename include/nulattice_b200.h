@@ -72,6 +72,8 @@ typedef struct {
                                      bits 4-7 lattice Lambda row pass, FP32 (0 256x2, 1 512x1);
                                      bits 8-15 Lambda column-pass row chunks (0: automatic);
                                      bits 16-19 lattice T2 kernel, FP64 (0 512x1, 1 256x1);
+                                     bits 20-23 not read (the Python tuner keeps the Lambda shapes of
+                                       the one-label problem there);
                                      bits 24-31 alike labels m (0 or 1: every label is stored).  m > 1:
                                        the m labels have the same tables, ladders and amplitudes, and
                                        every pair of labels the same exchange-symmetric t2; the problem

@@ -200,7 +200,8 @@ class _Instance:
 
     def item(self):
         it = _lib.BatchItem()
-        self.work.tune = self.eng.tune
+        if self.work is not self.eng:
+            self.eng.reduced()   # the word of one label
         it.prob = ctypes.pointer(self.work.prob)
         it.f32 = self.f32["state"]
         it.f64 = self.f64["state"]

@@ -171,7 +171,8 @@ class StructuredEngine:
             self.cache["reduced"] = red
         red = self.cache["reduced"]
         if red is not None:
-            red.tune = self.tune
+            from .tune import label_word
+            red.tune = label_word(self.tune)
             if self._prob is not None:
                 for name in ("uniform_nh", "diag_ladders", "max_fpp_offdiag"):
                     setattr(red.prob, name, getattr(self._prob, name))

@@ -7,6 +7,11 @@ column pass's row chunks), selected by the problem's ``tune`` word
 problem's own buffers with CUDA events, keeps the fastest, writes the word
 into the problem and caches it per GPU and problem shape in a JSON file
 (``$NLB_TUNE_CACHE``, default ``~/.cache/nulattice_b200/tune.json``).
+
+Alike labels: a Lambda run may have one label or every label stored, a sixth
+of the blocks or all of them, so the word holds the Lambda shapes of both
+(bits 4-15, and bits 20-23 for one label).  The forward shapes are those of
+every label; the two kernels of a step on one label have no choices.
 """
 from __future__ import annotations
 
@@ -27,8 +32,18 @@ FWD_F64 = {0: "512x1", 1: "256x1"}
 LAM_F32 = {0: "256x2", 1: "512x1"}
 
 
-def word(fwd32=0, lam32=0, chunks=0, fwd64=0):
-    return (fwd32 & 15) | ((lam32 & 15) << 4) | ((chunks & 255) << 8) | ((fwd64 & 15) << 16)
+def word(fwd32=0, lam32=0, chunks=0, fwd64=0, label=None):
+    """The tuning word; ``label``: (lam32, chunks) of a Lambda run on one
+    label, those of every label by default."""
+    one, rows = (lam32, chunks) if label is None else label
+    code = (one & 1) << 3 | (min(int(rows), 8).bit_length() & 7)      # chunks 0, 1, 2, 4, 8 (rounded down)
+    return (fwd32 & 15) | ((lam32 & 15) << 4) | ((chunks & 255) << 8) | ((fwd64 & 15) << 16) | code << 20
+
+
+def label_word(w):
+    """The word of the problem of one label: its Lambda shapes in their place."""
+    code = (w >> 20) & 15
+    return (w & 0xf000f) | (code >> 3) << 4 | (1 << (code & 7) >> 1) << 8
 
 
 def known_word(eng):
@@ -36,8 +51,7 @@ def known_word(eng):
     shape on this GPU if :func:`tune` stored one, else the shapes it picks
     on B200 at L=6, A=28 (two-row T2 kernel with 384 threads, Lambda column
     pass in two row chunks).  Non-lattice problems: 0 (no choices)."""
-    L = _lib.lib()
-    if not L.nlb_lambda_lattice((eng.reduced() or eng).prob):
+    if not _lib.lib().nlb_lambda_lattice(_built(eng)):
         return 0
     path = _cache_path()
     if os.path.exists(path):
@@ -52,9 +66,16 @@ def known_word(eng):
     return word(fwd32=6, chunks=chunks)
 
 
+def _built(eng):
+    """A problem of ``eng`` to ask about its kind: its own if it is built, else
+    the one of one label (which the solves of alike labels build anyway)."""
+    return eng.prob if eng._prob is not None else (eng.reduced() or eng).prob
+
+
 def describe(w):
     return {"t2_fp32": FWD_F32.get(w & 15), "lambda_fp32": LAM_F32.get((w >> 4) & 15),
-            "lambda_chunks": (w >> 8) & 255 or "auto", "t2_fp64": FWD_F64.get((w >> 16) & 15)}
+            "lambda_chunks": (w >> 8) & 255 or "auto", "t2_fp64": FWD_F64.get((w >> 16) & 15),
+            "label_lambda_fp32": LAM_F32.get((w >> 23) & 1), "label_chunks": (label_word(w) >> 8) & 255 or "auto"}
 
 
 def t2_kernel_fp32(w):
@@ -72,11 +93,10 @@ def _cache_path():
 
 
 def _key(eng):
-    work = eng.reduced() or eng
-    pl, nh = work.plan, work.prob.uniform_nh
+    pl, red = eng.plan, eng.reduced()
     name = torch.cuda.get_device_name(eng.dev)
-    alike = f"|alike={work.labels}" if work.labels > 1 else ""
-    return f"{name}|p={pl.p}|h={pl.h}|n_t2={pl.n_t2}|nh={nh}|ch={len(pl.channels)}{alike}"
+    alike = f"|alike={red.labels}" if red is not None else ""
+    return f"{name}|p={pl.p}|h={pl.h}|n_t2={pl.n_t2}|nh={_built(eng).uniform_nh}|ch={len(pl.channels)}{alike}"
 
 
 def _time(fn, reps):
@@ -91,6 +111,47 @@ def _time(fn, reps):
     return statistics.median(ts)
 
 
+def _some_steps(eng, code):
+    """Buffers with the amplitudes of three steps at parity 1 (never written by
+    the T2 stage that is timed after them)."""
+    L, dev = _lib.lib(), eng.dev
+    sp = ctypes_void(torch.cuda.current_stream(dev).cuda_stream)
+    t1 = _mp2_t1(eng.f_pp_np, eng.f_ph_np, eng.f_hh_np, 0.0)
+    e0 = eng.labels * float(np.sum(eng.f_ph_np * t1))
+    b = eng.buffers(code, 0)
+    b["t1"][0].copy_(torch.as_tensor(np.ascontiguousarray(t1).reshape(-1), device=dev))
+    b["t2"][0].zero_()
+    _lib.check(L.nlb_struct_ctrl_init(b["ctrl"].data_ptr(), 0.0, 0.5, 1 << 30, _lib.NLB_CRIT_SOA, 0, 0, e0, sp),
+               "ctrl_init")
+    for _ in range(3):
+        _lib.check(L.nlb_struct_step(eng.prob, b["state"], sp), "step")
+    return b
+
+
+def _tune_lambda(eng, reps, times, name):
+    """(row-pass shape, column-pass chunks) of the fastest FP32 Lambda step."""
+    from .adjoint import LambdaSolver
+    L = _lib.lib()
+    sp = ctypes_void(torch.cuda.current_stream(eng.dev).cuda_stream)
+    b32 = _some_steps(eng, _lib.NLB_F32)
+    b = LambdaSolver(eng).buffers(_lib.NLB_F32, 0)
+    b["t1"].copy_(b32["t1"][1])
+    b["t2"].copy_(b32["t2"][1])
+    cands = [0] + [c for c in (2, 4, 8) if c * 4 <= max(ch.np1 for ch in eng.plan.channels)]
+    res = {}
+    for lv in LAM_F32:
+        for c in cands:
+            eng.tune = word(lam32=lv, chunks=c)
+            _lib.check(L.nlb_lambda_init(eng.prob, b["state"], 0.0, 0.5, 1 << 30, 0, 0, sp), "lambda_init")
+
+            def run():
+                _lib.check(L.nlb_lambda_step(eng.prob, b["state"], sp), "lambda_step")
+            run()
+            res[(lv, c)] = _time(run, reps)
+    times[name] = {f"{LAM_F32[lv]}/chunks={c or 'auto'}": round(t * 1e3, 1) for (lv, c), t in res.items()}
+    return min(res, key=res.get)
+
+
 def tune(eng, lam=True, reps=7, use_cache=True, info=None):
     """Choose the launch shapes for engine ``eng`` and set ``eng.prob.tune``.
 
@@ -98,11 +159,10 @@ def tune(eng, lam=True, reps=7, use_cache=True, info=None):
     the defaults.  Returns the tuning word."""
     L = _lib.lib()
     info = {} if info is None else info
-    full, eng = eng, eng.reduced() or eng     # the shapes are timed on the problem that runs
     if not L.nlb_lambda_lattice(eng.prob):
-        full.tune = 0
+        eng.tune = 0
         return 0
-    key = _key(full)
+    key = _key(eng)
     path = _cache_path()
     cache = {}
     if use_cache and os.path.exists(path):
@@ -111,24 +171,14 @@ def tune(eng, lam=True, reps=7, use_cache=True, info=None):
         except (OSError, ValueError):
             cache = {}
     if use_cache and key in cache:
-        full.tune = int(cache[key]["word"])
+        eng.tune = int(cache[key]["word"])
         info.update(cache[key], cached=True)
-        return full.tune
-    dev = eng.dev
-    sp = ctypes_void(torch.cuda.current_stream(dev).cuda_stream)
-    pl = eng.plan
-    t1 = torch.as_tensor(_mp2_t1(eng.f_pp_np, eng.f_ph_np, eng.f_hh_np, 0.0).reshape(-1), device=dev)
-    e0 = float(np.sum(eng.f_ph_np.reshape(-1) * t1.cpu().numpy()))
+        return eng.tune
+    sp = ctypes_void(torch.cuda.current_stream(eng.dev).cuda_stream)
     times = {}
     best = {}
     for code, variants, shift, name in ((_lib.NLB_F32, FWD_F32, 0, "t2_fp32"), (_lib.NLB_F64, FWD_F64, 16, "t2_fp64")):
-        b = eng.buffers(code, 0)
-        b["t1"][0].copy_(t1)
-        b["t2"][0].zero_()
-        _lib.check(L.nlb_struct_ctrl_init(b["ctrl"].data_ptr(), 0.0, 0.5, 1 << 30, _lib.NLB_CRIT_SOA, 0, 0, e0, sp),
-                   "ctrl_init")
-        for _ in range(3):   # a few real steps: realistic amplitudes
-            _lib.check(L.nlb_struct_step(eng.prob, b["state"], sp), "step")
+        b = _some_steps(eng, code)
         res = {}
         for v in variants:
             eng.tune = v << shift
@@ -139,29 +189,14 @@ def tune(eng, lam=True, reps=7, use_cache=True, info=None):
             res[v] = _time(run, reps)
         best[name] = min(res, key=res.get)
         times[name] = {variants[v]: round(res[v] * 1e3, 1) for v in res}
-    lam32, chunks = 0, 0
+    every = one = (0, 0)
     if lam:
-        from .adjoint import LambdaSolver
-        solver = LambdaSolver(eng)
-        b = solver.buffers(_lib.NLB_F32, 0)
-        b32 = eng.buffers(_lib.NLB_F32, 0)
-        b["t1"].copy_(b32["t1"][0])
-        b["t2"].copy_(b32["t2"][0])
-        cands = [0] + [c for c in (2, 4, 8, 16, 32) if c * 4 <= max(ch.np1 for ch in pl.channels)]
-        res = {}
-        for lv in LAM_F32:
-            for c in cands:
-                eng.tune = word(lam32=lv, chunks=c)
-                _lib.check(L.nlb_lambda_init(eng.prob, b["state"], 0.0, 0.5, 1 << 30, 0, 0, sp), "lambda_init")
-
-                def run():
-                    _lib.check(L.nlb_lambda_step(eng.prob, b["state"], sp), "lambda_step")
-                run()
-                res[(lv, c)] = _time(run, reps)
-        lam32, chunks = min(res, key=res.get)
-        times["lambda_fp32"] = {f"{LAM_F32[lv]}/chunks={c or 'auto'}": round(t * 1e3, 1) for (lv, c), t in res.items()}
-    w = word(fwd32=best["t2_fp32"], lam32=lam32, chunks=chunks, fwd64=best["t2_fp64"])
-    full.tune = eng.tune = w
+        red = eng.reduced()
+        if red is not None:
+            one = _tune_lambda(red, reps, times, "label_lambda_fp32")
+        every = _tune_lambda(eng, reps, times, "lambda_fp32")
+    w = word(best["t2_fp32"], *every, best["t2_fp64"], label=one if eng.reduced() is not None else every)
+    eng.tune = w
     entry = {"word": w, "choice": describe(w), "us": times}
     info.update(entry, cached=False)
     if use_cache:

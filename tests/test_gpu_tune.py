@@ -59,3 +59,52 @@ def test_tuner_picks_a_valid_word(tmp_path, monkeypatch):
     eng2 = _engine()
     info2 = {}
     assert T.tune(eng2, info=info2) == w and info2["cached"]
+
+
+def test_tuner_times_the_shapes_it_names(tmp_path, monkeypatch):
+    """Every forward shape is timed on the problem whose kernels read it (every
+    label stored: four launches a step), the Lambda shapes on both problems, from
+    amplitudes of whole steps."""
+    monkeypatch.setenv("NLB_TUNE_CACHE", str(tmp_path / "tune.json"))
+    lib, stages, inits = T._lib.lib(), [], []
+
+    class Spy:
+        def __getattr__(self, name):
+            return getattr(lib, name)
+
+        def nlb_struct_stage(self, prob, st, stage, sp):
+            assert stage == T._lib.NLB_STAGE_T2 and lib.nlb_struct_step_launches(prob, st.dtype) == 4
+            stages.append((st.dtype, int(prob.tune)))
+            return lib.nlb_struct_stage(prob, st, stage, sp)
+
+        def nlb_lambda_init(self, prob, *a):
+            inits.append((int(prob.tune) >> 24, int(prob.tune) & 0xffff0))
+            return lib.nlb_lambda_init(prob, *a)
+
+    monkeypatch.setattr(T._lib, "lib", Spy)
+    eng = _engine()
+    seen = []
+    buffers = A.LambdaSolver.buffers
+    monkeypatch.setattr(A.LambdaSolver, "buffers", lambda s, *a: seen.append(buffers(s, *a)) or seen[-1])
+    w = T.tune(eng)
+    assert {x for x in stages if x[0] == T._lib.NLB_F32} == {(T._lib.NLB_F32, v) for v in T.FWD_F32}
+    assert {x for x in stages if x[0] == T._lib.NLB_F64} == {(T._lib.NLB_F64, v << 16) for v in T.FWD_F64}
+    for labels in (0, 4):
+        assert {x[1] for x in inits if x[0] == labels} >= {T.word(lam32=v, chunks=c) & 0xffff0 for v in T.LAM_F32
+                                                           for c in (0, 2, 4, 8)}
+    _, t1, t2 = solve_structured(_engine(), eps=0.0, mixed_eps=0.0, maxSteps=3, max_diis=0, precision="mixed",
+                                 refine=False, t2_format="compact")
+    one, every = seen
+    assert one["t2"].numel() * 6 == every["t2"].numel() == t2.numel()
+    for b in (one["t2"], every["t2"]):
+        np.testing.assert_allclose(b.cpu().numpy(), t2[:b.numel()].cpu().numpy(), atol=1e-5 * float(t2.abs().max()))
+    assert eng.tune == w and eng.reduced().tune == T.label_word(w)
+
+
+@pytest.mark.parametrize("label", [(0, 0), (1, 0), (0, 2), (1, 8)])
+def test_word_keeps_the_shapes_of_one_label(label):
+    w = T.word(fwd32=6, lam32=1, chunks=4, fwd64=1, label=label)
+    assert T.label_word(w) == T.word(fwd32=6, lam32=label[0], chunks=label[1], fwd64=1) & 0xfffff
+    assert T.describe(w)["label_chunks"] == (label[1] or "auto") and T.describe(w)["lambda_chunks"] == 4
+    # one choice for both, unless told apart
+    assert T.label_word(T.word(lam32=1, chunks=4)) == T.word(lam32=1, chunks=4) & 0xfffff
