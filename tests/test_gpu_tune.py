@@ -108,3 +108,11 @@ def test_word_keeps_the_shapes_of_one_label(label):
     assert T.describe(w)["label_chunks"] == (label[1] or "auto") and T.describe(w)["lambda_chunks"] == 4
     # one choice for both, unless told apart
     assert T.label_word(T.word(lam32=1, chunks=4)) == T.word(lam32=1, chunks=4) & 0xfffff
+
+
+def test_untuned_word_leaves_the_chunks_of_one_label_to_the_kernel(tmp_path, monkeypatch):
+    """Two row chunks are the choice for six channels; one has a sixth of the blocks."""
+    monkeypatch.setenv("NLB_TUNE_CACHE", str(tmp_path / "none.json"))
+    eng = _engine()
+    eng.prob.tune = T.known_word(eng)
+    assert (eng.prob.tune >> 8) & 255 == 2 and (eng.reduced().prob.tune >> 8) & 255 == 0
