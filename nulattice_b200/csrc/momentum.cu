@@ -130,12 +130,15 @@ __global__ void k_pw_init(nlb_pw_problem P, double* t2, double delta) {
 // entries of one momentum block (their rows repeat every 16 nc amplitudes, so a
 // warp reads 32 neighbours of one pa), its warps over the row groups pa; the
 // eight partial sums are added in warp order.  A lane per pa read one amplitude
-// of every 32-byte sector: 19.5 us for A=28 L=6 FP64, 8.9 us this way.
+// of every 32-byte sector: 19.5 us for A=28 L=6 FP64, 8.9 us this way.  Sums in
+// FP64 for either type: a warp's run of npa / 8 terms grows with the lattice, and
+// FP32 runs left nine FP32 steps of A=4 L=6 8.2e-8 off (mean of 12 couplings)
+// against 6.9e-8 (3.2 -> 3.7 us for A=4 L=5, the nine steps as long as before).
 constexpr int kPwMEntries = 32;
 
 template <typename F>
 __global__ void __launch_bounds__(256) k_pw_M(nlb_pw_problem P, const F* __restrict__ t2, F* __restrict__ M) {
-    __shared__ F part[8][kPwMEntries];
+    __shared__ double part[8][kPwMEntries];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t n = P.n_m / kPwMEntries;   // 16 nc entries per block, nc a multiple of 16: no remainder
     for (int64_t u = blockIdx.x; u < n; u += gridDim.x) {
@@ -144,16 +147,16 @@ __global__ void __launch_bounds__(256) k_pw_M(nlb_pw_problem P, const F* __restr
         const int npa = P.blk_nr[b] >> 4;
         const int64_t step = (int64_t)16 * P.blk_nc[b];
         const F* T = t2 + P.blk_off[b] + (e - P.m_off[b]);
-        F acc = 0.0;
+        double acc = 0.0;
 #pragma unroll 4
-        for (int pa = w; pa < npa; pa += 8) acc += T[pa * step];
+        for (int pa = w; pa < npa; pa += 8) acc += (double)T[pa * step];
         part[w][lane] = acc;
         __syncthreads();
         if (w == 0) {
-            F m = part[0][lane];
+            double m = part[0][lane];
 #pragma unroll
             for (int k = 1; k < 8; ++k) m += part[k][lane];
-            M[e] = m;
+            M[e] = (F)m;
         }
         __syncthreads();
     }

@@ -146,3 +146,21 @@ def test_steps_with_more_holes_than_a_group_of_lanes(precision, eps):
         want = MM.step(plan, V, fpp, fhh, want)
     assert np.abs(want - got[0]).max() > 1e-3 * np.abs(want).max()
     assert np.abs(got[1] - want).max() <= 2 * 8 * 304 * eps * np.abs(want).max()
+
+
+@pytest.mark.parametrize("L,A", [(2, 4), (3, 28), (5, 4), (6, 28)])
+def test_sums_over_particle_momenta_round_once(L, A):
+    """M of FP32 amplitudes: FP64 sums, rounded to FP32 at the end."""
+    plan, eng, args = _engine(L, A, -6.0, -6.0, 1.0)
+    e32 = MB.MomentumEngine(plan, *args, DEV, dtype=torch.float32, tables=eng)
+    t2 = torch.randn(plan.n_t2, generator=torch.Generator("cuda").manual_seed(3), device=DEV)
+    e32.energy(t2)
+    got, x = e32.bufs["M"].cpu().numpy()[:int(e32.P.n_m)], t2.double().cpu().numpy()
+    at = 0
+    for b, (nr, nc) in enumerate(zip(plan.nr, plan.nc)):
+        block = x[int(plan.blk_off[b]):int(plan.blk_off[b + 1])].reshape(nr // 16, 16 * nc)
+        want, size = block.sum(0), np.abs(block).sum(0)
+        # one rounding to 24 bits, and those of the FP64 sum
+        assert np.all(np.abs(got[at:at + 16 * nc] - want) <= 2.0 ** -24 * np.abs(want) + nr * 2.0 ** -53 * size)
+        at += 16 * nc
+    assert at == len(got)
