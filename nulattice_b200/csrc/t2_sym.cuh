@@ -219,15 +219,15 @@ __global__ void __launch_bounds__(kSymMost * sym_parts<T>(NH), sizeof(T) == 4 ? 
     }
     // T1 update of (a, i): R1 = f_ph + F2 of every other label + X_pp t1 + t1
     // X_hh with F2 = sum_k Gb[k][i,k] (coupled_cluster.py:342-414), by the last
-    // threads (the first have a column each)
+    // threads (the first have a column each); F2 is added in FP64 for either type
     if (run == 0 && nt - 1 - tid < NH) {
         const int i = nt - 1 - tid;
-        T f2 = T(0);
+        double f2 = 0.0;
         if (t2) {
 #pragma unroll
-            for (int k = 0; k < NH; ++k) f2 += sgb[(k * NH + i) * 8 + k];
+            for (int k = 0; k < NH; ++k) f2 += (double)sgb[(k * NH + i) * 8 + k];
         }
-        double h1 = sfh[i] + sym_others(P) * (double)f2;
+        double h1 = sfh[i] + sym_others(P) * f2;
 #pragma unroll
         for (int q = 0; q <= kSymNf; ++q) h1 += sft[q * NH + i];
 #pragma unroll

@@ -297,3 +297,37 @@ def test_amplitudes_count_as_alike_bit_for_bit(dtype, step):
         y = t1.clone()
         y[plan.p_of[0][1], plan.h_of[0][0]] = float("nan")
         assert red.compress(y, t2) is None
+
+
+def _one_step(red, t1, t2, code):
+    """One step on one label from (t1, t2): the next (t1, t2)."""
+    lib, sp = _lib.lib(), torch.cuda.current_stream().cuda_stream
+    assert lib.nlb_struct_step_launches(red.prob, code) == 2
+    b = red.buffers(code, 0)
+    b["t1"][0].copy_(torch.as_tensor(t1.ravel()))
+    b["t2"][0].copy_(torch.as_tensor(t2.ravel()))
+    _lib.check(lib.nlb_struct_ctrl_init(b["ctrl"].data_ptr(), 0.0, 0.5, 10, _lib.NLB_CRIT_SOA, 0, 0, 0.0, sp), "init")
+    _lib.check(lib.nlb_struct_step(red.prob, b["state"], sp), "step")
+    return b["t1"][1].cpu().numpy().reshape(t1.shape), b["t2"][1].double().cpu().numpy().reshape(t2.shape)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("code", [_lib.NLB_F32, _lib.NLB_F64])
+def test_t1_adds_the_holes_of_its_t2_term_in_fp64(code):
+    """Holes whose terms 1, 2^-26 and -1 leave 2^-26: lost where they are added in
+    FP32.  t1 = 0, so a step is t1 = (1 - m) (f_ph + 3 F2) / -(f_aa - f_ii)."""
+    _, eng = _engine(3, 3)
+    red = eng.reduced()
+    n, h = red.plan.p, red.plan.h
+    t2 = np.zeros((n, n, h, h))
+    ptr, col, val = (np.asarray(x) for x in (red.plan.fph_ptr, red.plan.fph_col, red.plan.fph_val))
+    # a particle next to each hole alone
+    near = [next(int(c) for c in col[ptr[k]:ptr[k + 1]] if np.sum(col == c) == 1) for k in range(h)]
+    a = next(x for x in range(n) if x not in near)
+    for k, x in enumerate((1.0, 2.0 ** -26, -1.0)):
+        f = float(val[ptr[k]:ptr[k + 1]][col[ptr[k]:ptr[k + 1]] == near[k]][0])
+        t2[a, near[k], :, k] = x / f
+    t2 += t2.transpose(1, 0, 3, 2)                        # exchange-symmetric
+    t1, _ = _one_step(red, np.zeros((n, h)), t2, code)
+    want = 0.5 * (red.f_ph_np[a] + 3 * 2.0 ** -26) / (np.diag(red.f_hh_np) - red.f_pp_np[a, a])
+    np.testing.assert_allclose(t1[a], want, rtol=0, atol=1e-14)
