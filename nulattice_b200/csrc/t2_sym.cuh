@@ -148,8 +148,7 @@ __global__ void __launch_bounds__(kSymMost * sym_parts<T>(NH), sizeof(T) == 4 ? 
         }
         if (tid == nt - 1) {
             s_sum = s_entry(P, t1, ga);
-            reinterpret_cast<T*>(V.dXp2)[a] = (T)P.fpp_diag[ga];   // for the update pass
-            reinterpret_cast<T*>(V.dXp1)[a] = (T)s_sum;
+            V.dpc[a] = P.fpp_diag[ga] - s_sum;   // for the update pass
         }
     }
     if (tid < NH) {
@@ -338,9 +337,8 @@ __device__ void sym_update_body(const nlb_struct_problem& P, const nlb_struct_st
     // a thread owns one hole pair (i, j) of every CPB-th column
     constexpr int CPB = kThreads / NHP;
     const int cl = threadIdx.x / NHP, hp = threadIdx.x - cl * NHP, i = hp / NH, j = hp - i * NH;
-    const T* dp = reinterpret_cast<const T*>(V.dXp2);
-    const T* sp = reinterpret_cast<const T*>(V.dXp1);
-    const T da = dp[a], sa = sp[a], dh = (T)(V.dhc[i] + V.dhc[j]);
+    // denominators: the diagonals of X_pp and X_hh added in FP64 and rounded once
+    const double da = V.dpc[a] + (V.dhc[i] + V.dhc[j]);
     T nrm = T(0);
     if (cl < CPB) {
         int64_t e0 = ((int64_t)a * np + b0 + cl) * NHP + hp;              // (a, b, i, j)
@@ -349,7 +347,7 @@ __device__ void sym_update_body(const nlb_struct_problem& P, const nlb_struct_st
         // kSymU columns whose loads go out together
         for (int b = b0 + cl; b < b1; b += kSymU * CPB) {
             T x[kSymU], s1[kSymU], s2[kSymU];
-            T db[kSymU], sb[kSymU];
+            double db[kSymU];
 #pragma unroll
             for (int u = 0; u < kSymU; ++u) {
                 const int bu = b + u * CPB;
@@ -357,16 +355,15 @@ __device__ void sym_update_body(const nlb_struct_problem& P, const nlb_struct_st
                 x[u] = B[e0 + u * CPB * NHP];
                 s1[u] = __ldcg(Bo + e0 + u * CPB * NHP);
                 s2[u] = __ldcg(Bo + x0 + u * xs);
-                db[u] = dp[bu];
-                sb[u] = sp[bu];
+                db[u] = V.dpc[bu];
             }
 #pragma unroll
             for (int u = 0; u < kSymU; ++u) {
                 const int bu = b + u * CPB;
                 // (i, j) of column a stands for (j, i), too
                 if (bu >= b1 || (bu == a && i > j)) continue;
-                const T d0 = da + db[u] + dh, r = s1[u] + s2[u];
-                const T tn = x[u] - lat_div(r, d0 - (sa + sb[u]));
+                const T r = s1[u] + s2[u];
+                const T tn = x[u] - lat_div(r, (T)(da + db[u]));
                 const T out = m * x[u] + om * tn, d = out - x[u];
                 const bool two = bu != a || i != j;   // two places, and twice in the norm
                 nrm += (two ? T(2) : T(1)) * d * d;

@@ -331,3 +331,31 @@ def test_t1_adds_the_holes_of_its_t2_term_in_fp64(code):
     t1, _ = _one_step(red, np.zeros((n, h)), t2, code)
     want = 0.5 * (red.f_ph_np[a] + 3 * 2.0 ** -26) / (np.diag(red.f_hh_np) - red.f_pp_np[a, a])
     np.testing.assert_allclose(t1[a], want, rtol=0, atol=1e-14)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("code,eps", [(_lib.NLB_F32, 2.0 ** -24), (_lib.NLB_F64, 2.0 ** -53)])
+def test_denominators_round_once(code, eps):
+    """Diagonals of 1e6 in f_pp and f_hh whose sums leave a few units.  t2 = 0, so a
+    step is t2 = (1 - m) R / D with R the ladders on t1 t1; its error is that of R
+    (two products and a sum), of D (one rounding), of the quotient (2 ulp) and of
+    the update, D's FP64 terms and the FP64 sums over f_ph t1 aside."""
+    _, eng = _engine(4, 3)
+    f = [eng.f_pp_np + 1e6 * np.eye(eng.plan.p), eng.f_ph_np, eng.f_hh_np + 1e6 * np.eye(eng.plan.h)]
+    _, _, two = _inputs(4, 3)
+    plan, _ = S.detect(f, two)
+    red = StructuredEngine(plan, f, torch.device("cuda:0")).reduced()
+    n, h = red.plan.p, red.plan.h
+    t1 = 0.01 * np.random.default_rng(1).standard_normal((n, h))
+    _, t2 = _one_step(red, t1, np.zeros((n, n, h, h)), code)
+    pp, hh = np.zeros(n * n), np.zeros(h * h)
+    pp[np.diff(red.plan.pp_ptr[0]) > 0], hh[np.diff(red.plan.hh_ptr[0]) > 0] = red.plan.pp_val[0], red.plan.hh_val[0]
+    R = (pp.reshape(n, n)[:, :, None, None] + hh.reshape(h, h)) * t1[:, None, :, None] * t1[None, :, None, :]
+    dp = np.diag(red.f_pp_np) - (red.f_ph_np * t1).sum(1)
+    dh = -np.diag(red.f_hh_np) - (red.f_ph_np * t1).sum(0)
+    D = -((dp[:, None, None, None] + dp[None, :, None, None]) + (dh[:, None] + dh[None, :]))
+    want = 0.5 * R / D
+    assert np.abs(D).max() < 100 and np.abs(want).max() > 0
+    # 4e6 * 2^-53 from the FP64 additions of the diagonals, against the smallest |D|
+    lim = 10 * eps + 4 * 4e6 * 2.0 ** -53 / np.abs(D).min()
+    assert np.all(np.abs(t2 - want) <= lim * np.abs(want))
