@@ -143,7 +143,7 @@ class _Instance:
         plan, why = _structure.detect(fock, two)
         if plan is None:
             raise ValueError(f"instance (A={A}, L={L}) needs the structured engine: {why}")
-        self.eng = StructuredEngine(plan, fock, dev)
+        self.eng = StructuredEngine(plan, fock, dev, defer=True)
         # alike labels: the instance runs on one of them
         solver = None
         eng = self.eng.reduced()

@@ -101,13 +101,16 @@ class StructuredEngine:
 
     When the labels are alike (:func:`structure.alike_labels`), the work runs
     on :meth:`reduced`, the engine of one label and one channel, and the
-    results are written out in the full layout; the tables of the full
-    problem are then built when something asks for them (``prob``).
+    results are written out in the full layout.
 
     ``labels``: how many alike labels a one-label plan stands for.
+    ``defer``: leave the device tables to the first use of ``prob`` (a solve
+    on one label needs none of the full problem's); otherwise they are
+    uploaded here, and ``prob`` can be used where nothing may be allocated,
+    as inside a stream capture.
     """
 
-    def __init__(self, plan, fock_mats, device, labels=1):
+    def __init__(self, plan, fock_mats, device, labels=1, defer=False):
         self.plan = plan
         self.dev = device
         self.labels = labels
@@ -123,10 +126,12 @@ class StructuredEngine:
         self._bufs = {}
         self.cache = {}
         self.launches = 0
+        if not defer:
+            self._build()
 
     @property
     def prob(self):
-        """The device problem (:c:type:`nlb_struct_problem`), built on first use."""
+        """The device problem (:c:type:`nlb_struct_problem`)."""
         if self._prob is None:
             self._build()
         return self._prob
@@ -163,7 +168,7 @@ class StructuredEngine:
                 one, m = got
                 P0, H0 = self.plan.p_of[0], self.plan.h_of[0]
                 red = StructuredEngine(one, [self.f_pp_np[np.ix_(P0, P0)], self.f_ph_np[np.ix_(P0, H0)],
-                                             self.f_hh_np[np.ix_(H0, H0)]], self.dev, labels=m)
+                                             self.f_hh_np[np.ix_(H0, H0)]], self.dev, labels=m, defer=True)
                 cat = lambda xs: torch.as_tensor(np.concatenate(xs).astype(np.int32), device=self.dev)  # noqa: E731
                 red.orders = cat(self.plan.p_of), cat(self.plan.h_of)
                 red.sizes = self.plan.p, self.plan.h
@@ -613,7 +618,7 @@ def ccsd_solver(fock_mats, two_body_int, t1initial=None, eps=1e-8, maxSteps=1000
     else:
         info["engine"] = "structured"
         t0 = time.perf_counter()
-        eng = StructuredEngine(plan, fock_mats, dev)
+        eng = StructuredEngine(plan, fock_mats, dev, defer=True)   # used here alone
         from . import tune as _tune
         eng.tune = _tune.known_word(eng)   # cached or default launch shapes, no timing
         info["t_engine"] = time.perf_counter() - t0

@@ -54,7 +54,7 @@ def known_word(eng):
     and FP64 multipliers takes 97 and 135 us against 101 and 143 us in two
     chunks, at L=5 61 and 69 against 68 and 81 us).  Non-lattice problems: 0
     (no choices)."""
-    if not _lib.lib().nlb_lambda_lattice(_built(eng)):
+    if not _lib.lib().nlb_lambda_lattice((eng.reduced() or eng).prob):
         return 0
     path = _cache_path()
     if os.path.exists(path):
@@ -67,12 +67,6 @@ def known_word(eng):
             pass
     chunks = 2 if max(ch.np1 for ch in eng.plan.channels) >= 8 else 0
     return word(fwd32=6, chunks=chunks, label=(0, 0))
-
-
-def _built(eng):
-    """A problem of ``eng`` to ask about its kind: its own if it is built, else
-    the one of one label (which the solves of alike labels build anyway)."""
-    return eng.prob if eng._prob is not None else (eng.reduced() or eng).prob
 
 
 def describe(w):
@@ -97,9 +91,10 @@ def _cache_path():
 
 def _key(eng):
     pl, red = eng.plan, eng.reduced()
+    nh = (red or eng).prob.uniform_nh
     name = torch.cuda.get_device_name(eng.dev)
     alike = f"|alike={red.labels}" if red is not None else ""
-    return f"{name}|p={pl.p}|h={pl.h}|n_t2={pl.n_t2}|nh={_built(eng).uniform_nh}|ch={len(pl.channels)}{alike}"
+    return f"{name}|p={pl.p}|h={pl.h}|n_t2={pl.n_t2}|nh={nh}|ch={len(pl.channels)}{alike}"
 
 
 def _time(fn, reps):

@@ -57,6 +57,16 @@ def test_labels_that_differ_are_not_alike(what):
     assert S.alike_labels(plan, fock[2]) is None
 
 
+def test_a_new_engine_has_its_tables():
+    """The device problem of an engine exists before anything asks for it: a
+    program may first use it inside a stream capture."""
+    _, fock, two = _inputs(3, 1)
+    plan, _ = S.detect(fock, two)
+    eng = StructuredEngine(plan, fock, torch.device("cpu"))
+    built = eng._prob
+    assert built is not None and built.p == plan.p and eng.prob is built
+
+
 def _engine(L, sites, full=False):
     holes, fock, two = _inputs(L, sites)
     plan, _ = S.detect(fock, two)
@@ -359,3 +369,31 @@ def test_denominators_round_once(code, eps):
     # 4e6 * 2^-53 from the FP64 additions of the diagonals, against the smallest |D|
     lim = 10 * eps + 4 * 4e6 * 2.0 ** -53 / np.abs(D).min()
     assert np.all(np.abs(t2 - want) <= lim * np.abs(want))
+
+
+@pytest.mark.gpu
+def test_a_new_engine_steps_inside_a_capture():
+    """Steps of a fresh engine's problem with the caller's buffers, captured: no
+    allocation in between, and the replay is the step."""
+    _, eng = _engine(3, 2)
+    lib = _lib.lib()
+    b = StructuredEngine(eng.plan, [eng.f_pp_np, eng.f_ph_np, eng.f_hh_np], eng.dev).buffers(_lib.NLB_F64, 0)
+    fresh = StructuredEngine(eng.plan, [eng.f_pp_np, eng.f_ph_np, eng.f_hh_np], eng.dev)
+    t1 = torch.as_tensor(eng.f_ph_np * 0.01).cuda()
+    out = []
+    for capture in (False, True):
+        b["t1"][0].copy_(t1.reshape(-1))
+        b["t2"][0].zero_()
+        sp = torch.cuda.current_stream().cuda_stream
+        _lib.check(lib.nlb_struct_ctrl_init(b["ctrl"].data_ptr(), 0.0, 0.5, 10, _lib.NLB_CRIT_SOA, 0, 0, 0.0, sp), "init")
+        if capture:
+            before = torch.cuda.memory_allocated()
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g):
+                _lib.check(lib.nlb_struct_step(fresh.prob, b["state"], torch.cuda.current_stream().cuda_stream), "step")
+                assert torch.cuda.memory_allocated() == before
+            g.replay()
+        else:
+            _lib.check(lib.nlb_struct_step(eng.prob, b["state"], sp), "step")
+        out.append((b["t1"][1].cpu(), b["t2"][1].cpu()))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
