@@ -27,6 +27,8 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <atomic>
+
 #include "nulattice_b200.h"
 
 static thread_local char g_err[512] = "";
@@ -1290,19 +1292,21 @@ int g_nocc = 0;
 
 int64_t smem_limit();
 
+// Raises a kernel's dynamic shared-memory limit to the device maximum (less its
+// static shared memory): the 48 KB default counts static shared memory too, and
+// lowering the limit for a smaller problem would break launches (and captured
+// graphs) of a larger one.
+void raise_smem(const void* fn) {
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, fn) == cudaSuccess)
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(smem_limit() - (int64_t)fa.sharedSizeBytes));
+}
+
 int blocks_per_sm(const void* fn, int64_t smem, int threads = kThreads) {
     for (int k = 0; k < g_nocc; ++k)
         if (g_occ[k].fn == fn && g_occ[k].smem == smem) return g_occ[k].bps;
-    // raise the limit to the device maximum (less the kernel's static shared
-    // memory) for every kernel that takes dynamic shared memory: the 48 KB
-    // default counts static shared memory too, and lowering the limit for a
-    // smaller problem would break launches (and captured graphs) of a larger one
-    if (smem > 0) {
-        cudaFuncAttributes fa;
-        if (cudaFuncGetAttributes(&fa, fn) == cudaSuccess)
-            cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(smem_limit() - (int64_t)fa.sharedSizeBytes));
-    }
+    if (smem > 0) raise_smem(fn);
     int bps = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, fn, threads, (size_t)smem) != cudaSuccess || bps <= 0)
         bps = 1;
@@ -1492,7 +1496,16 @@ struct SymRow {
         nc = nc * PARTS < 128 ? (128 / PARTS + 31) / 32 * 32 : nc;   // the staging and the tables want threads, too
         const int nt = nc * PARTS;
         const int64_t sm = sym_smem<T, NH>(P->p, nc).total;
-        blocks_per_sm(reinterpret_cast<const void*>(kern), sm, nt);   // raises the shared-memory limit
+        // once per kernel and device, whatever the size: an entry of the occupancy
+        // table for every problem size would fill it
+        static std::atomic<uint64_t> raised{0};
+        int dev = 0;
+        cudaGetDevice(&dev);
+        const uint64_t bit = dev < 64 ? uint64_t(1) << dev : 0;
+        if (!(raised.load(std::memory_order_relaxed) & bit)) {
+            raise_smem(reinterpret_cast<const void*>(kern));
+            raised.fetch_or(bit, std::memory_order_relaxed);
+        }
         kern<<<(unsigned)(P->p * runs), nt, (size_t)sm, st>>>(*P, *S, runs);
         return 0;
     }

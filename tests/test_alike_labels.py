@@ -397,3 +397,25 @@ def test_a_new_engine_steps_inside_a_capture():
             _lib.check(lib.nlb_struct_step(eng.prob, b["state"], sp), "step")
         out.append((b["t1"][1].cpu(), b["t2"][1].cpu()))
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
+@pytest.mark.gpu
+def test_launches_ask_for_attributes_once_per_kernel():
+    """After steps of seventy problem sizes a step is its two launches and nothing
+    else: no table of launch attributes is full."""
+    from torch.profiler import ProfilerActivity, profile
+    lib, sp = _lib.lib(), torch.cuda.current_stream().cuda_stream
+    for L in (2, 3, 4, 5, 6):
+        for sites in range(1, 8):
+            _, fock, two = _inputs(L, sites)
+            plan, _ = S.detect(fock, two)
+            red = StructuredEngine(plan, fock, torch.device("cuda:0")).reduced()
+            for code in (_lib.NLB_F32, _lib.NLB_F64):
+                _one_step(red, np.zeros((red.plan.p, red.plan.h)), np.zeros(red.plan.n_t2), code)
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
+        for _ in range(3):
+            _lib.check(lib.nlb_struct_step(red.prob, red.buffers(_lib.NLB_F64, 0)["state"], sp), "step")
+        torch.cuda.synchronize()
+    calls = [e.name for e in prof.events()]
+    assert sum(x == "cudaLaunchKernel" for x in calls) == 6
+    assert not [x for x in calls if "Attribute" in x or "Occupancy" in x]
