@@ -263,9 +263,8 @@ def test_derivative_that_treats_labels_differently(L, sites):
     np.testing.assert_allclose(grads[0], grads[1], rtol=1e-9)
 
 
-def _labels(fock, two, keep):
-    """The inputs of some of the labels: Fock blocks and ladders of their states."""
-    plan, _ = S.detect(fock, two)
+def _labels(plan, fock, two, keep):
+    """The inputs of some of a plan's labels: Fock blocks and ladders of their states."""
     P, H = (np.flatnonzero(np.isin(x, keep)) for x in (plan.p_label, plan.h_label))
     ladders = []
     for block, states in ((two[0], P), (two[5], H)):
@@ -283,7 +282,7 @@ def test_amplitudes_count_as_alike_bit_for_bit(dtype, step):
     are each seen, also where two labels leave one block and no copy to compare."""
     holes, fock, two = _inputs(3, 3)
     for keep in ([0, 1, 2, 3], [0, 1]):
-        f, t = _labels(fock, two, keep)
+        f, t = _labels(S.detect(fock, two)[0], fock, two, keep)
         plan, why = S.detect(f, t)
         eng = StructuredEngine(plan, f, torch.device("cuda:0"))
         red = eng.reduced()
@@ -419,3 +418,67 @@ def test_launches_ask_for_attributes_once_per_kernel():
     calls = [e.name for e in prof.events()]
     assert sum(x == "cudaLaunchKernel" for x in calls) == 6
     assert not [x for x in calls if "Attribute" in x or "Occupancy" in x]
+
+
+NINE = SEVEN + [(1, 1, 0), (1, -1, 0)]
+
+
+def _exchange_hops(plan, strength):
+    """v_pppp that moves a pair (x, y) of any two labels to (y, x), for some x, y."""
+    rows = []
+    for g in range(plan.n_labels):
+        for k in range(plan.n_labels):
+            for x, y in ((0, 1), (1, 0), (2, 5), (5, 2)):
+                if g != k:
+                    a, b, c, d = plan.p_of[g][x], plan.p_of[k][y], plan.p_of[g][y], plan.p_of[k][x]
+                    rows += [(a, b, c, d, strength), (b, a, c, d, -strength)]
+    return np.array(rows)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,sites,keep,hops", [(3, 3, (0, 1), 0), (3, 3, (0, 2, 3), 0), (4, 7, (1, 2), 0),
+                                               (4, 7, (0, 1, 3), 0), (4, 9, (0, 1, 2, 3), 0), (3, 8, (0, 1, 2), 0),
+                                               (3, 2, (0, 1, 2, 3), 0.3), (4, 7, (0, 1), 0.3), (4, 9, (0, 1, 2), 0.3)])
+def test_other_alike_problems(L, sites, keep, hops):
+    """Two and three labels, more than seven holes, ladders that are not diagonal:
+    steps, a converged solve and (diagonal ladders) gradients on one label against
+    every label stored."""
+    holes = [[x % L, y % L, z % L, t, s] for (x, y, z) in NINE[:sites] for t in (0, 1) for s in (0, 1)]
+    v, w = ham.contact_couplings(-3.1, 0.9)
+    _, fock, two = ham.normal_ordered_hamiltonian(L, holes, v, v, w, dense=False)
+    plan, _ = S.detect(fock, two)
+    prob = A.lattice_problem(L, holes)
+    derivs = [(de, *_labels(plan, df, dt, keep)) for de, df, dt in (prob.dv, prob.dw)]
+    fock, two = _labels(plan, fock, two, keep)
+    if hops:
+        part, _ = S.detect(fock, two)
+        idx, val = two[0]
+        extra = _exchange_hops(part, hops)
+        two[0] = np.concatenate([idx, extra[:, :4]]).astype(np.int64), np.concatenate([val, extra[:, 4]])
+    plan, why = S.detect(fock, two)
+    assert plan is not None, why
+    out, start = {}, None
+    for full in (False, True):
+        eng = StructuredEngine(plan, fock, torch.device("cuda:0"))
+        assert bool(eng.prob.diag_ladders) == (not hops)
+        if full:
+            eng.cache["reduced"] = None
+        else:
+            assert eng.reduced().labels == len(keep)
+        for precision, fmt in (("fp64", "dense"), ("fp64", "compact"), ("mixed", "compact")):
+            e, t1, t2 = solve_structured(eng, eps=0.0, mixed_eps=0.0, maxSteps=4, max_diis=0, refine=False,
+                                         precision=precision, t2_format=fmt)
+            out[full, precision, fmt] = e, t1.cpu().numpy(), t2.double().cpu().numpy()
+        info = {}
+        e, t1, t2 = solve_structured(eng, eps=1e-13, maxSteps=2000, max_diis=8, t2_format="compact", info=info)
+        assert info["status"] == "converged"
+        out[full, "converged"] = e, t1.cpu().numpy(), t2.cpu().numpy()
+        start = (t1, t2) if start is None else start
+        if not hops:
+            out[full, "gradient"] = A.lambda_gradient(eng, *start, derivs, tol=1e-11, precision="fp64")
+    for key, got in out.items():
+        if key[0]:
+            continue
+        lim = {"converged": 1e-7, "gradient": 1e-9, "fp64": 1e-13, "mixed": 4e-6}[key[1]]
+        for x, y in zip(got, out[(True,) + key[1:]]):
+            assert np.abs(np.asarray(x) - y).max() <= lim * np.abs(y).max(), key

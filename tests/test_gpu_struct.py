@@ -4,7 +4,7 @@ import pytest
 import torch
 
 import golden_io as G
-from nulattice_b200 import ccsd_solver
+from nulattice_b200 import _lib, ccsd_solver
 from nulattice_b200 import hamiltonian as ham
 from oracle import ccsd_oracle as O
 
@@ -168,6 +168,8 @@ def _lattice_engine(L, A, general=False):
     plan, why = S.detect(fock, two)
     assert plan is not None, why
     eng = StructuredEngine(plan, fock, torch.device(DEV))
+    eng.cache["reduced"] = None   # every label stored: one label has kernels of its own
+    assert all(_lib.lib().nlb_struct_step_launches(eng.prob, code) == 4 for code in (_lib.NLB_F32, _lib.NLB_F64))
     assert eng.prob.uniform_nh == 7 and eng.prob.diag_ladders and eng.prob.max_fpp_offdiag == 6
     if general:
         eng.prob.max_fpp_offdiag = 99   # the one-hole-pair-per-thread lattice kernel no longer applies
@@ -202,6 +204,7 @@ def _lattice_vs_general(L, precision, tol, shape):
         info = {}
         e, t1, t2 = solve_structured(eng, eps=0.0, maxSteps=11, max_diis=4, precision=precision,
                                      mixed_eps=0.0, refine=False, t2_format="compact", info=info)
+        assert info["n_t2_stored"] == eng.plan.n_t2
         out.append((e, t1.cpu().numpy(), t2.double().cpu().numpy()))
     (ea, t1a, t2a), (eb, t1b, t2b) = out
     assert np.abs(t2a).max() > 1e-4

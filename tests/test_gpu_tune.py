@@ -26,6 +26,8 @@ def test_forward_launch_shapes_agree(precision, tol):
     words = [T.word(fwd32=v) for v in T.FWD_F32] if precision == "mixed" else [T.word(fwd64=v) for v in T.FWD_F64]
     for w in words:
         eng = _engine()
+        eng.cache["reduced"] = None   # every label stored: one label has kernels of its own
+        assert all(T._lib.lib().nlb_struct_step_launches(eng.prob, c) == 4 for c in (T._lib.NLB_F32, T._lib.NLB_F64))
         eng.prob.tune = w
         e, t1, t2 = solve_structured(eng, eps=0.0, maxSteps=9, max_diis=4, precision=precision, mixed_eps=0.0,
                                      refine=False, t2_format="compact")
@@ -40,7 +42,9 @@ def test_lambda_launch_shapes_agree():
     e, t1, t2c = solve_structured(eng, eps=1e-12, maxSteps=2000, max_diis=8, t2_format="compact")
     prob = A.lattice_problem(4, ham.closed_shell_holes(4, 28))
     ref = None
-    for w in (T.word(), T.word(lam32=1), T.word(chunks=2), T.word(lam32=1, chunks=4)):
+    for k, w in enumerate(2 * [T.word(), T.word(lam32=1), T.word(chunks=2), T.word(lam32=1, chunks=4)]):
+        if k == 4:
+            eng.cache["reduced"] = None   # one label, then every label stored
         eng.prob.tune = w
         g = A.lambda_gradient(eng, t1, t2c, [prob.dv, prob.dw], tol=1e-10, precision="mixed")
         if ref is None:
