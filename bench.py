@@ -667,11 +667,11 @@ def batch_leg(dev, peak_gbs, rank=0, ws=1):
     t_batch = gmax(t_batch)
     res = scan.results()
     ok = [r for r in res if r["status"] == "converged" and r["lambda_status"] == "converged"]
-    # algorithmic bytes of the steps that ran: 3 passes over the compact T2
+    # algorithmic bytes of the steps that ran: 3 passes over the stored T2
     # (read, write, DIIS error) per forward or Lambda step, FP32 or FP64
     alg = 0.0
     for r in res:
-        n2 = r["n_t2"]
+        n2 = r["n_t2_stored"]
         alg += 3 * n2 * (4 * r["mixed_iterations"] + 8 * (r["iterations"] - r["mixed_iterations"]))
         alg += 3 * n2 * 6 * r["lambda_iterations"]   # FP32 and FP64 Lambda steps, ~6 bytes on average
     # one at a time: the batch's algorithm and plain FP64 Jacobi, on the same engines

@@ -260,7 +260,9 @@ class BatchScan:
         _lib.check(_lib.lib().nlb_batch_launch(self.handle, ctypes_void(stream.cuda_stream)), "batch_launch")
 
     def results(self):
-        """Per-instance results after a launch has finished."""
+        """Per-instance results after a launch has finished.  ``n_t2``: compact
+        amplitudes of the problem; ``n_t2_stored``: those the instance stores
+        (one channel when its labels are alike)."""
         res = []
         status = {0: "running", 1: "converged", 2: "max_iter", 3: "diverged"}
         for x in self.instances:
@@ -276,7 +278,8 @@ class BatchScan:
             res.append(dict(A=x.A, L=x.L, C2=x.C2, C3=x.C3, E=float(o[0]) + x.e_ref, E_corr=float(o[0]),
                             dE_dC2=grads[0], dE_dC3=grads[1], status=status.get(int(o[3]), "?"),
                             lambda_status=status.get(int(o[5]), "?"), iterations=int(o[4]),
-                            mixed_iterations=int(o[7]), lambda_iterations=int(o[6]), n_t2=x.eng.plan.n_t2))
+                            mixed_iterations=int(o[7]), lambda_iterations=int(o[6]), n_t2=x.eng.plan.n_t2,
+                            n_t2_stored=x.work.plan.n_t2))
         return res
 
     def close(self):

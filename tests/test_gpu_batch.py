@@ -33,6 +33,8 @@ def test_batch_matches_single_instance_pipeline():
         assert r["E"] == pytest.approx(E, rel=1e-8), (r, E)
         assert r["dE_dC2"] == pytest.approx(g2, rel=1e-6), (r, g2)
         assert r["dE_dC3"] == pytest.approx(g3, rel=1e-6), (r, g3)
+        # the size of the problem, and what the instance holds and moves: one label's channel of six
+        assert r["n_t2"] == 6 * r["n_t2_stored"] == info["n_t2"]
         # the FP32 phase stops near its noise floor (1e-8), so its length can
         # differ between runs; both pipelines end converged in FP64
         assert r["iterations"] > 0 and info["iterations"] > 0
