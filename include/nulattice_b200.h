@@ -115,7 +115,9 @@ typedef struct {
     double e_last;      /* energy of the last finished step */
     double eps;
     double mixing;
-    double gram[121];   /* DIIS Gram matrix (max_diis <= 10), then coefficients */
+    double gram[121];   /* DIIS Gram matrix (max_diis <= 10), then coefficients; the last entry (not
+                           one of a Gram matrix) counts the finished blocks of a step on one label and
+                           is zero between steps */
     int32_t parity;     /* which amplitude buffer is current */
     int32_t iter;
     int32_t status;

@@ -1035,7 +1035,7 @@ __global__ void __launch_bounds__(kThreads) k_diis_reduce(nlb_ctrl* c, const dou
 __global__ void k_diis_solve(nlb_ctrl* c) {
     // One warp.  Lane t owns column t of the bordered matrix in shared memory,
     // and finds the pivot and the factors as row t: one division and
-    // three barriers per column (a division and two barriers per row: 13.0 us
+    // four barriers per column (a division and two barriers per row: 13.0 us
     // at eight vectors, all latency; 10.8 us this way, most of it the serial
     // back substitution, whose order stays).  Every entry sees the same
     // operations in the same order as a serial elimination (partial pivoting,

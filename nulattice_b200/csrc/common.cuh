@@ -302,17 +302,6 @@ __device__ __forceinline__ void lds8(const int32_t* p, int (&v)[8]) {
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
-
-// Four consecutive shared-memory values (16-byte aligned) with vector loads.
-__device__ __forceinline__ void lds4(const float* p, float (&v)[4]) {
-    const float4 a = *reinterpret_cast<const float4*>(p);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-}
-__device__ __forceinline__ void lds4(const double* p, double (&v)[4]) {
-    const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
-
 // Jacobi quotient R / D.  FP32 amplitudes: the approximate reciprocal (the
 // denominators only set the step length, the fixed point R = 0 does not
 // depend on them); FP64: IEEE division.

@@ -8,9 +8,10 @@
 // rank-h part of X_pp along b, X_hh along j) and half of the ladders and of the
 // diagonal, which act on both.  The half diagonal comes first in the sum, so
 // that S stays small near the solution and FP32 keeps its digits (relative
-// error of nine FP32 steps against FP64, rms over 12 couplings each at L=3-5:
-// 6.4-7.9e-8; with the diagonal added at the end 8.0-12e-8; a residual summed
-// whole 6.3-9.4e-8).  S of a row needs only that row:
+// error of nine FP32 steps against FP64, rms over 12 couplings each at L=3-6 and
+// two, three and seven sites: 6.4-7.9e-8, 7.1e-8 on average; a residual summed
+// whole, with every label stored, 6.3-7.8e-8 and 7.2e-8; with the diagonal added
+// at the end 8.0-12e-8).  S of a row needs only that row:
 //
 // * k_sym_row: S of each row a into the output buffer, and the T1 update of
 //   particle a (its T1 Fock term needs only the row, too);
