@@ -93,6 +93,13 @@ def _upload(arrays, device):
             for name, a in arrays.items()}
 
 
+def label_word(w):
+    """The tuning word of the problem of one label: of the whole word, its
+    Lambda shapes (bits 20-23, see :mod:`tune`) in their place."""
+    code = (w >> 20) & 15
+    return (w & 0xf000f) | (code >> 3) << 4 | (1 << (code & 7) >> 1) << 8
+
+
 class StructuredEngine:
     """Device tables and buffers of one structured problem.
 
@@ -176,7 +183,6 @@ class StructuredEngine:
             self.cache["reduced"] = red
         red = self.cache["reduced"]
         if red is not None:
-            from .tune import label_word
             red.tune = label_word(self.tune)
             if self._prob is not None:
                 for name in ("uniform_nh", "diag_ladders", "max_fpp_offdiag"):
@@ -303,12 +309,7 @@ class StructuredEngine:
         prob.p, prob.h, prob.n_labels, prob.n_channels = pl.p, pl.h, G, len(pl.channels)
         prob.n_t2, prob.n_g, prob.n_f2, prob.n_rows = pl.n_t2, self.n_g, self.n_f2, self.n_rows
         prob.n_t1c, prob.n_xc, prob.max_row, prob.max_nh = self.n_t1c, self.n_xc, self.max_row, self.max_nh
-        nhs = {(ch.nh1, ch.nh2) for ch in pl.channels}
-        uniform = 0
-        if len(nhs) == 1:
-            n1, n2 = next(iter(nhs))
-            uniform = n1 if n1 == n2 else 0
-        prob.uniform_nh = uniform
+        prob.uniform_nh = pl.uniform_nh
         # diagonal ladders: at most one entry per output pair, and it is the
         # pair itself (with counts of 0 or 1 the rows that hold an entry are
         # the non-zero counts, in order)
@@ -618,7 +619,11 @@ def ccsd_solver(fock_mats, two_body_int, t1initial=None, eps=1e-8, maxSteps=1000
     else:
         info["engine"] = "structured"
         t0 = time.perf_counter()
-        eng = StructuredEngine(plan, fock_mats, dev, defer=True)   # used here alone
+        # used here alone: a solve builds the tables it runs on and no others
+        me = float(mixed_eps) if mixed_eps is not None else max(float(eps), 1e-7)
+        eng = StructuredEngine(plan, fock_mats, dev, defer=True)
+        if _every_label(precision, True, _CRIT[criterion], max_diis, maxSteps, eps, me):
+            eng.cache["reduced"] = None
         from . import tune as _tune
         eng.tune = _tune.known_word(eng)   # cached or default launch shapes, no timing
         info["t_engine"] = time.perf_counter() - t0
@@ -644,6 +649,22 @@ def ccsd_solver(fock_mats, two_body_int, t1initial=None, eps=1e-8, maxSteps=1000
     return e, t1, t2
 
 
+def _every_label(precision, refine, crit, max_diis, max_steps, eps, mixed_eps):
+    """Whether a solve of alike labels keeps every one stored.
+
+    A mixed solve that converges in FP64 does when its FP32 phase can pulse.  Its
+    energy test passes by chance where the energy difference changes sign, at a step
+    that moves with every rounding before a pulse, and the amplitudes it leaves move
+    with it: over 120 couplings at L=3-6 (mixed_eps=1e-6, eps=1e-11) those of one
+    label and of every label were up to 1.5e-7 apart (4.5e-8 and 1.5e-7 from the
+    fixed point), which is more than such a solve may change by.  Without a pulse
+    they agree to 4e-13.  A solve whose answer is the FP32 phase's (eps no tighter
+    than mixed_eps, or refine=False) promises no such digits (both forms leave 1e-6,
+    at worst 3e-4, at mixed_eps=1e-8) and runs on one label."""
+    return (precision == "mixed" and refine and crit == _lib.NLB_CRIT_SOA and 0 < max_diis <= max_steps
+            and float(eps) < mixed_eps)
+
+
 def solve_structured(eng, t1initial=None, eps=1e-8, maxSteps=1000, max_diis=10, delta=0.0, mixing=0.5,
                      verbose=False, ccs=False, criterion="soa", precision="fp64", t2_format="dense",
                      mixed_eps=None, info=None, sync_every=16, t2_events=None, refine=True, loop="graph"):
@@ -655,21 +676,10 @@ def solve_structured(eng, t1initial=None, eps=1e-8, maxSteps=1000, max_diis=10, 
     the host, which costs no graph build and suits an engine used once."""
     info = {} if info is None else info
     L = _lib.lib()
-    full, red = eng, eng.reduced()
+    full = eng
     crit = _CRIT[criterion]
     me = float(mixed_eps) if mixed_eps is not None else max(float(eps), 1e-7)
-    # A mixed solve that converges in FP64 keeps every label stored when its FP32
-    # phase can pulse.  Its energy test passes by chance where the energy difference
-    # changes sign, at a step that moves with every rounding before a pulse, and the
-    # amplitudes it leaves move with it: over 120 couplings at L=3-6 (mixed_eps=1e-6,
-    # eps=1e-11) those of one label and of every label were up to 1.5e-7 apart
-    # (4.5e-8 and 1.5e-7 from the fixed point), which is more than such a solve may
-    # change by.  Without a pulse they agree to 4e-13.  A solve whose answer is the
-    # FP32 phase's (eps no tighter than mixed_eps, or refine=False) promises no such
-    # digits (both forms leave 1e-6, at worst 3e-4, at mixed_eps=1e-8) and runs on one
-    # label.
-    if precision == "mixed" and refine and crit == _lib.NLB_CRIT_SOA and 0 < max_diis <= maxSteps and float(eps) < me:
-        red = None
+    red = None if _every_label(precision, refine, crit, max_diis, maxSteps, eps, me) else eng.reduced()
     t1_start = None
     if t1initial is not None:
         t1_start = np.asarray(_np(t1initial), dtype=np.float64)

@@ -210,6 +210,12 @@ class ChannelPlan:
             t2[np.ix_(P2, P1, H2, H1)] = B.transpose(1, 0, 3, 2)
         return t2
 
+    @property
+    def uniform_nh(self):
+        """Holes of every label of a channel when all have as many, else 0."""
+        nhs = {n for ch in self.channels for n in (ch.nh1, ch.nh2)}
+        return nhs.pop() if len(nhs) == 1 else 0
+
     def t1_mask(self):
         return self.p_label[:, None] == self.h_label[None, :]
 

@@ -24,7 +24,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .ccsd import _mp2_t1, ctypes_void
+from .ccsd import _mp2_t1, ctypes_void, label_word
 
 FWD_F32 = {0: "256x2", 1: "512x1", 2: "384x1", 3: "512x1 x2", 4: "384x1 x2", 5: "rows2 256x1", 6: "rows2 384x1",
            7: "rows2 448x1", 8: "rows2 512x1"}
@@ -38,12 +38,6 @@ def word(fwd32=0, lam32=0, chunks=0, fwd64=0, label=None):
     one, rows = (lam32, chunks) if label is None else label
     code = (one & 1) << 3 | (min(int(rows), 8).bit_length() & 7)      # chunks 0, 1, 2, 4, 8 (rounded down)
     return (fwd32 & 15) | ((lam32 & 15) << 4) | ((chunks & 255) << 8) | ((fwd64 & 15) << 16) | code << 20
-
-
-def label_word(w):
-    """The word of the problem of one label: its Lambda shapes in their place."""
-    code = (w >> 20) & 15
-    return (w & 0xf000f) | (code >> 3) << 4 | (1 << (code & 7) >> 1) << 8
 
 
 def known_word(eng):
@@ -90,11 +84,9 @@ def _cache_path():
 
 
 def _key(eng):
-    pl, red = eng.plan, eng.reduced()
-    nh = (red or eng).prob.uniform_nh
+    pl = eng.plan
     name = torch.cuda.get_device_name(eng.dev)
-    alike = f"|alike={red.labels}" if red is not None else ""
-    return f"{name}|p={pl.p}|h={pl.h}|n_t2={pl.n_t2}|nh={nh}|ch={len(pl.channels)}{alike}"
+    return f"{name}|p={pl.p}|h={pl.h}|n_t2={pl.n_t2}|nh={pl.uniform_nh}|ch={len(pl.channels)}"
 
 
 def _time(fn, reps):
