@@ -276,10 +276,13 @@ def lambda_gradient(eng, t1_dev, t2c_dev, derivs, tol=1e-9, mixing=0.5, max_step
         # alike labels: everything on one of them, when the amplitudes and the
         # derivative Hamiltonians treat the labels alike, too
         solver = _kept_solver(red)
-        t2c_dev = t2c_dev.reshape(-1).contiguous()
+        t1_dev = t1_dev.to(device=red.dev, dtype=torch.float64).contiguous()
+        t2c_dev = t2c_dev.to(red.dev).reshape(-1).contiguous()
+        if t2c_dev.dtype != torch.float32:
+            t2c_dev = t2c_dev.to(torch.float64)
         t1 = None
         if all(solver.coefficients(dfock, dtwo) is not None for _, dfock, dtwo in derivs):
-            t1 = red.compress(t1_dev.to(torch.float64).contiguous(), t2c_dev)
+            t1 = red.compress(t1_dev, t2c_dev)
         if t1 is not None:
             eng, t1_dev, t2c_dev = red, t1, t2c_dev[:red.plan.n_t2]
     pl, dev = eng.plan, eng.dev

@@ -220,6 +220,14 @@ class StructuredEngine:
         compact) have the alike-label form -- labels and exchange bit for bit, as
         the steps of one label leave them -- else None.  The first block of
         ``t2_full`` is then t2."""
+        P, H = self.sizes
+        pairs = self.labels * (self.labels - 1) // 2
+        for name, x, n, kinds in (("t1", t1_full, P * H, (torch.float64,)),
+                                  ("t2", t2_full, pairs * self.plan.n_t2, (torch.float64, torch.float32))):
+            here = x.device.type == self.dev.type and self.dev.index in (None, x.device.index)
+            if not here or x.dtype not in kinds or x.numel() != n or not x.is_contiguous():
+                raise ValueError(f"{name}: {n} contiguous amplitudes on {self.dev} expected, got "
+                                 f"{tuple(x.shape)} {x.dtype} on {x.device}")
         t1 = torch.empty(self.plan.p * self.plan.h, dtype=torch.float64, device=self.dev)
         out = torch.empty(3, dtype=torch.int64, device=self.dev)
         code = _lib.NLB_F32 if t2_full.dtype == torch.float32 else _lib.NLB_F64
@@ -683,6 +691,8 @@ def solve_structured(eng, t1initial=None, eps=1e-8, maxSteps=1000, max_diis=10, 
     t1_start = None
     if t1initial is not None:
         t1_start = np.asarray(_np(t1initial), dtype=np.float64)
+        if t1_start.shape != full.f_ph_np.shape:
+            raise ValueError(f"t1initial: shape {full.f_ph_np.shape} expected, got {t1_start.shape}")
         if red is not None:   # one label only when the start has the form
             blocks = [t1_start[np.ix_(P, H)] for P, H in zip(full.plan.p_of, full.plan.h_of)]
             alike = all(np.array_equal(blocks[0], x) for x in blocks[1:]) and \

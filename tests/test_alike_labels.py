@@ -482,3 +482,28 @@ def test_other_alike_problems(L, sites, keep, hops):
         lim = {"converged": 1e-7, "gradient": 1e-9, "fp64": 1e-13, "mixed": 4e-6}[key[1]]
         for x, y in zip(got, out[(True,) + key[1:]]):
             assert np.abs(np.asarray(x) - y).max() <= lim * np.abs(y).max(), key
+
+
+@pytest.mark.gpu
+def test_amplitudes_from_the_host_and_of_a_wrong_size():
+    """A gradient takes amplitudes from wherever they are, and refuses those that are
+    not the engine's; a start of another shape is refused, too."""
+    holes, fock, two = _inputs(3, 3)
+    plan, _ = S.detect(fock, two)
+    prob = A.lattice_problem(3, holes)
+    kw = dict(tol=1e-10, precision="fp64")
+    want = None
+    for device in ("cuda", "cuda:0"):
+        eng = StructuredEngine(plan, fock, torch.device(device))
+        _, t1, t2 = solve_structured(eng, eps=1e-13, max_diis=8, maxSteps=2000, t2_format="compact")
+        got = A.lambda_gradient(eng, t1, t2, [prob.dv], **kw)
+        want = want or got
+        assert got == want
+    for x, y in ((t1.cpu(), t2.cpu()), (t1.reshape(-1), t2.reshape(6, -1)), (t1.t().contiguous().t(), t2.cpu())):
+        assert A.lambda_gradient(eng, x, y, [prob.dv], **kw) == want
+    for x, y in ((t1, t2[:-1]), (t1, t2[:t2.numel() // 6]), (t1[:-1], t2), (t1, torch.cat([t2, t2]))):
+        with pytest.raises((ValueError, RuntimeError)):
+            A.lambda_gradient(eng, x, y, [prob.dv], **kw)
+    for shape in ((eng.plan.p + 1, eng.plan.h), (eng.plan.p, eng.plan.h + 2), (1, eng.plan.h)):
+        with pytest.raises(ValueError):
+            solve_structured(eng, t1initial=np.zeros(shape), eps=0.0, maxSteps=2)
