@@ -89,12 +89,14 @@ class LambdaSolver:
     multipliers, U, T and control block are written out in the layout of the
     full buffers."""
 
-    # fewest particles of a label for a run on one label: below, a step is
-    # launches only and the check of the amplitudes and the copies in and out
-    # cost more than they save (eight steps on one B200, one label against all:
-    # 20 particles, 7 sites 546 and 506 us; 26, 1 site 567 and 588 us; 57, 7
-    # sites 688 and 862 us; 124, 1 site 891 and 1564 us)
-    label_from = 24
+    # fewest particles of a label for a run on one label.  The check of the
+    # amplitudes and the copies in and out are about 100 us a run, a step gains
+    # more with more particles: runs of one, four and nine steps on one B200, one
+    # label (all labels), us: 26 particles, 1 site FP64 214 (112), 363 (306), 633
+    # (651); 57, 7 sites FP32 221 (142), 382 (387), 651 (786) and FP64 230 (159),
+    # 421 (466), 710 (951); 118, 7 sites FP32 245 (210), 447 (638), 769 (1362).
+    # The line is where four steps break even.
+    label_from = 48
 
     def __init__(self, eng):
         L = _lib.lib()

@@ -183,6 +183,7 @@ def test_lambda_steps_on_one_label(L, sites, code, tol):
         if not full:
             start = t1, t2
         solver = A.LambdaSolver(eng)
+        solver.label_from = 1    # small labels, too
         b = solver.buffers(code, 0)
         b["t1"].copy_(start[0].reshape(-1))
         b["t2"].copy_(start[1])
@@ -243,7 +244,7 @@ def test_lambda_pulse_extrapolates_every_entry(L, sites, code, eps):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("L,sites", [(3, 3), (4, 7)])
+@pytest.mark.parametrize("L,sites", [(4, 3), (4, 7)])
 def test_derivative_that_treats_labels_differently(L, sites):
     """Alike amplitudes and a derivative Hamiltonian with one pair of labels apart:
     the multipliers may run on one label, the coupling sums take all of them."""
@@ -507,3 +508,18 @@ def test_amplitudes_from_the_host_and_of_a_wrong_size():
     for shape in ((eng.plan.p + 1, eng.plan.h), (eng.plan.p, eng.plan.h + 2), (1, eng.plan.h)):
         with pytest.raises(ValueError):
             solve_structured(eng, t1initial=np.zeros(shape), eps=0.0, maxSteps=2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,sites,one", [(3, 1, False), (3, 7, False), (4, 7, True)])
+def test_short_lambda_runs_of_small_labels_keep_every_label(L, sites, one):
+    """The check and the copies of a run on one label cost more than four steps of
+    some twenty particles gain."""
+    _, eng = _engine(L, sites)
+    _, t1, t2 = solve_structured(eng, eps=1e-12, max_diis=8, t2_format="compact")
+    solver = A.LambdaSolver(eng)
+    b = solver.buffers(_lib.NLB_F64, 0)
+    b["t1"].copy_(t1.reshape(-1))
+    b["t2"].copy_(t2)
+    solver.run(b, 0.0, 0.5, 4, 0, False)
+    assert (solver._label is not None) == one
