@@ -194,6 +194,10 @@ class LambdaSolver:
         label = self._alike(b, keep)
         if label is not None:
             return self._run_label(label, b, tol, mixing, max_steps, max_diis, keep)
+        return self._run_all(b, tol, mixing, max_steps, max_diis, keep)
+
+    def _run_all(self, b, tol, mixing, max_steps, max_diis, keep):
+        """:meth:`run` with every label that the engine stores."""
         L = _lib.lib()
         dev = self.eng.dev
         stream = torch.cuda.current_stream(dev)
@@ -223,12 +227,14 @@ class LambdaSolver:
     def _alike(self, b, keep):
         """(one-label solver, its start) when the amplitudes of ``b`` (and the
         multipliers, if kept) have the alike-label form, else None."""
-        red = self.eng.reduced()
-        if red is None or red.plan.p < self.label_from:
+        if len(self.eng.plan.p_of[0]) < self.label_from:
             return None
-        t1 = red.compress(b["t1"], b["t2"])
-        lam1 = red.compress(b["lam1"][0], b["lam2"][0]) if keep and t1 is not None else None
-        if t1 is None or (keep and lam1 is None):
+        got = self.eng.alike_amplitudes(b["t1"], b["t2"])
+        if got is None:
+            return None
+        red, t1 = got
+        lam1 = red.compress(b["lam1"][0], b["lam2"][0]) if keep else None
+        if keep and lam1 is None:
             return None
         if self._label is None:
             self._label = LambdaSolver(red)
@@ -271,21 +277,21 @@ def lambda_gradient(eng, t1_dev, t2c_dev, derivs, tol=1e-9, mixing=0.5, max_step
     subspace (0: plain Jacobi with mixing)."""
     info = {} if info is None else info
     L = _lib.lib()
-    red = eng.reduced()
-    if not (red or eng).prob.diag_ladders:
+    t1_dev = t1_dev.to(device=eng.dev, dtype=torch.float64).contiguous()
+    t2c_dev = t2c_dev.to(eng.dev).reshape(-1).contiguous()
+    if t2c_dev.dtype != torch.float32:
+        t2c_dev = t2c_dev.to(torch.float64)
+    # alike labels: everything on one of them, when the amplitudes and the
+    # derivative Hamiltonians treat the labels alike, too
+    got = eng.alike_amplitudes(t1_dev, t2c_dev)
+    if not (eng if got is None else got[0]).prob.diag_ladders:
         raise ValueError("the adjoint needs diagonal ladders (SU(4) closed-site inputs)")
-    if red is not None:
-        # alike labels: everything on one of them, when the amplitudes and the
-        # derivative Hamiltonians treat the labels alike, too
+    run = LambdaSolver._run_all
+    if got is not None:
+        red, t1 = got
         solver = _kept_solver(red)
-        t1_dev = t1_dev.to(device=red.dev, dtype=torch.float64).contiguous()
-        t2c_dev = t2c_dev.to(red.dev).reshape(-1).contiguous()
-        if t2c_dev.dtype != torch.float32:
-            t2c_dev = t2c_dev.to(torch.float64)
-        t1 = None
+        run = LambdaSolver.run       # amplitudes alike, the derivatives perhaps not
         if all(solver.coefficients(dfock, dtwo) is not None for _, dfock, dtwo in derivs):
-            t1 = red.compress(t1_dev, t2c_dev)
-        if t1 is not None:
             eng, t1_dev, t2c_dev = red, t1, t2c_dev[:red.plan.n_t2]
     pl, dev = eng.plan, eng.dev
     sp = ctypes_void(torch.cuda.current_stream(dev).cuda_stream)
@@ -304,7 +310,7 @@ def lambda_gradient(eng, t1_dev, t2c_dev, derivs, tol=1e-9, mixing=0.5, max_step
         b32 = solver.buffers(_lib.NLB_F32, max_diis)
         b32["t1"].copy_(t1_dev.reshape(-1))
         b32["t2"].copy_(t2c_dev.reshape(-1).to(torch.float32))
-        c = solver.run(b32, max(tol, tol_fp32), mixing, max_steps, max_diis, keep=False)
+        c = run(solver, b32, max(tol, tol_fp32), mixing, max_steps, max_diis, keep=False)
         iters += c.iter
         launches += solver.launches
         info["lambda_iters_fp32"] = c.iter
@@ -319,7 +325,7 @@ def lambda_gradient(eng, t1_dev, t2c_dev, derivs, tol=1e-9, mixing=0.5, max_step
     # instead of eight steps (the equations are linear)
     diis64 = min(max_diis, 4) if keep else max_diis
     t1 = time.perf_counter()
-    c = solver.run(b64, tol, mixing, max(max_steps - iters, 1), diis64, keep=keep)
+    c = run(solver, b64, tol, mixing, max(max_steps - iters, 1), diis64, keep=keep)
     iters += c.iter
     launches += solver.launches
     info["t_lambda_fp64"] = time.perf_counter() - t1
@@ -398,7 +404,7 @@ def ccsd_energy_and_gradient(L, holes, C2, C3, device="cuda:0", precision="fp64"
             raise ValueError(f"the adjoint needs the structured engine: {why}")
         engine = StructuredEngine(plan, fock, dev)
         from . import tune as _tune
-        engine.tune = _tune.known_word(engine)
+        engine.tune = _tune.known_word(engine, engine.prob)
     eng = info["engine"] = engine
     torch.cuda.synchronize(dev)
     t0 = time.perf_counter()

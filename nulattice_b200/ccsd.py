@@ -238,6 +238,21 @@ class StructuredEngine:
         o = out.cpu().numpy()
         return t1 if o[0] == 0 and o[1] == 0 else None
 
+    def alike_amplitudes(self, t1, t2):
+        """(engine of one label, its t1) when amplitudes of the full layout
+        have the alike-label form (:meth:`compress`), else None.  Amplitudes
+        whose first two blocks begin differently, as those of a solve on every
+        label do, are told apart before the engine of one label is built."""
+        chs = self.plan.channels
+        if "reduced" not in self.cache and len(chs) > 1:
+            n, k = chs[0].size, min(chs[0].size, 1024)
+            # (copies to the host: a comparison on the device would allocate)
+            if chs[1].size != n or not torch.equal(t2[:k].cpu(), t2[n:n + k].cpu()):
+                return None
+        red = self.reduced()
+        one = None if red is None else red.compress(t1, t2)
+        return None if one is None else (red, one)
+
     def _build(self):
         pl = self.plan
         f_pp, f_ph, f_hh = self.f_pp_np, self.f_ph_np, self.f_hh_np

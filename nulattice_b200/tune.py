@@ -40,15 +40,16 @@ def word(fwd32=0, lam32=0, chunks=0, fwd64=0, label=None):
     return (fwd32 & 15) | ((lam32 & 15) << 4) | ((chunks & 255) << 8) | ((fwd64 & 15) << 16) | code << 20
 
 
-def known_word(eng):
+def known_word(eng, prob=None):
     """Launch shapes without timing: the cached word of ``eng``'s problem
     shape on this GPU if :func:`tune` stored one, else the shapes it picks
     on B200 at L=6, A=28 (two-row T2 kernel with 384 threads, Lambda column
     pass in two row chunks; on one label the automatic count: a step of FP32
     and FP64 multipliers takes 97 and 135 us against 101 and 143 us in two
     chunks, at L=5 61 and 69 against 68 and 81 us).  Non-lattice problems: 0
-    (no choices)."""
-    if not _lib.lib().nlb_lambda_lattice((eng.reduced() or eng).prob):
+    (no choices).  ``prob``: a problem of ``eng`` that is built (by default
+    the one of one label, which the solves of alike labels run on)."""
+    if not _lib.lib().nlb_lambda_lattice(prob if prob is not None else (eng.reduced() or eng).prob):
         return 0
     path = _cache_path()
     if os.path.exists(path):

@@ -523,3 +523,14 @@ def test_short_lambda_runs_of_small_labels_keep_every_label(L, sites, one):
     b["t2"].copy_(t2)
     solver.run(b, 0.0, 0.5, 4, 0, False)
     assert (solver._label is not None) == one
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision,one", [("mixed", False), ("fp64", True)])
+def test_gradients_build_the_engine_they_run_on(precision, one):
+    """A mixed gradient runs on every label from start to end; nothing of the
+    problem of one label is made for it."""
+    holes = [[0, 0, 0, t, s] for t in (0, 1) for s in (0, 1)]
+    info = {}
+    A.ccsd_energy_and_gradient(3, holes, -3.1, 0.9, precision=precision, eps=1e-11, lambda_tol=1e-9, info=info)
+    assert ("reduced" in info["engine"].cache) == one
