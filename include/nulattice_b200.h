@@ -208,9 +208,12 @@ int64_t nlb_struct_noalloc_scratch_bytes(const nlb_struct_problem *prob, int32_t
 
 /* Pulsed DIIS of the torch solver (CCM/soa/coupled_cluster.py:522-567): when
  * ctrl->diis_pulse is set, build the Gram matrix of the stored error vectors
- * (FP64), solve the bordered system in FP64 on the device and extrapolate the
+ * (FP64; FP32 vectors of every label: FP32 products and per-thread sums),
+ * solve the bordered system in FP64 on the device and extrapolate the
  * current amplitudes in place.  No-op otherwise.  `max_diis` must equal the
  * value given to nlb_struct_ctrl_init (it selects the compiled kernel).
+ * Label-symmetric problems: t2 and the rings as nlb_struct_step leaves them
+ * (the pairs a <= b are read and written in both places).
  * Reads t1, t2, the rings, ctrl and the partial-sum area of st->prep; st->g
  * and st->f2 are not used. */
 int nlb_struct_diis(const nlb_struct_problem *prob, const nlb_struct_state *st, int32_t max_diis,
